@@ -1490,18 +1490,23 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
         if (!grid_sync(gb, B, bar_target)) return;
     }
 
-    // sum over the grid of the block partials (a, b) written at `part`
-    auto grid_totals = [&](double a, double b, double& ta, double& tb) -> bool {
+    // sum over the grid of the block partials (a, b), published in slot
+    // `slot` of `part`.  The two reductions of an iteration use two slots: a
+    // block past the first one's barrier may publish its second partials
+    // while a late block still reads the first ones; with a barrier between
+    // two uses of a slot no block can overwrite what another still reads.
+    auto grid_totals = [&](int slot, double a, double b, double& ta, double& tb) -> bool {
+        double* pt = part + size_t(slot) * 2 * B;
         block_sum2(a, b, sh);
         if (threadIdx.x == 0) {
-            part[2 * blockIdx.x] = a;
-            part[2 * blockIdx.x + 1] = b;
+            pt[2 * blockIdx.x] = a;
+            pt[2 * blockIdx.x + 1] = b;
         }
         if (!grid_sync(gb, B, bar_target)) return false;
         double x = 0.0, y = 0.0;
         for (int k = threadIdx.x; k < int(B); k += PB) {
-            x += __ldcg(part + 2 * k);
-            y += __ldcg(part + 2 * k + 1);
+            x += __ldcg(pt + 2 * k);
+            y += __ldcg(pt + 2 * k + 1);
         }
         block_sum2(x, y, sh);
         ta = x;
@@ -1587,7 +1592,7 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
         double pq = 0.0, zero = 0.0;
         for (int t = threadIdx.x; t < rows; t += PB) pq += p_s[t] * q_s[t];
         double pap, unused;
-        if (!grid_totals(pq, zero, pap, unused)) return;
+        if (!grid_totals(0, pq, zero, pap, unused)) return;
         if (!(pap > 0.0)) {  // p.Kp <= 0 or NaN: breakdown
             it += 1;
             if (writer) s->pap = pap;
@@ -1608,7 +1613,7 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
             lrz += ri * zi;
         }
         double rr, rz_new;
-        if (!grid_totals(lrr, lrz, rr, rz_new)) return;
+        if (!grid_totals(1, lrr, lrz, rr, rz_new)) return;
         it += 1;
         const double res = sqrt(rr) / s_c[0];
         if (threadIdx.x == 0) {
@@ -2569,7 +2574,7 @@ struct PcgRun {
             if (!fn) return -1;
             DBuf<double> part, z;
             DBuf<GridBarrier> gb;
-            part.alloc(ctx->pool, 2 * size_t(B) + 2);
+            part.alloc(ctx->pool, 4 * size_t(B) + 2);  // two slots of pairs
             z.alloc(ctx->pool, n + 1);
             gb.alloc(ctx->pool, 1);
             SVX_CUDA(cudaMemsetAsync(gb.p, 0, sizeof(GridBarrier), st));
