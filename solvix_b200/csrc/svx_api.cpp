@@ -966,6 +966,14 @@ int svx_ctx_create(int device, svx_ctx_t** out) {
         if (const char* e = std::getenv("SVX_PCG_ALG")) ctx->pcg_alg = (e[0] == '0') ? 0 : 1;
         if (const char* e = std::getenv("SVX_PCG_STAGE")) ctx->pcg_stage = (e[0] != '0');
         if (const char* e = std::getenv("SVX_FP32_QUADS")) ctx->fp32_quads = (e[0] != '0');
+        if (const char* e = std::getenv("SVX_RESIDENT")) ctx->resident = (e[0] != '0');
+        auto nodes_env = [](const char* name, int& to) {
+            const char* e = std::getenv(name);
+            const int v = e ? std::atoi(e) : 0;
+            if (v >= 32 && v <= 512 && v % 32 == 0) to = v;
+        };
+        nodes_env("SVX_RESIDENT_NODES", ctx->resident_nodes_single);
+        nodes_env("SVX_RESIDENT_BATCH_NODES", ctx->resident_nodes_batch);
         if (const char* e = std::getenv("SVX_PCG_LANES")) ctx->pcg_lanes = std::atoi(e);
         if (const char* e = std::getenv("SVX_PCG_UNROLL")) {
             const long v = std::strtol(e, nullptr, 10);
@@ -1005,6 +1013,11 @@ int svx_ctx_destroy(svx_ctx_t* ctx) {
             cudaStreamSynchronize(x);
             cudaStreamDestroy(x);
         }
+    for (cudaStream_t x : ctx->class_streams) {
+        cudaStreamSynchronize(x);
+        cudaStreamDestroy(x);
+    }
+    for (cudaEvent_t e : ctx->class_events) cudaEventDestroy(e);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return SVX_OK;

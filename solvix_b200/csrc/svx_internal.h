@@ -199,6 +199,17 @@ struct svx_ctx {
     // 1: the three-barrier form stages the gathered p window in shared
     // memory; SVX_PCG_STAGE=0 gathers from L2 (measurements)
     int pcg_stage = 1;
+    // 1: plane models that fit run the chip-resident cluster kernel
+    // (svx_resident.cu); SVX_RESIDENT=0 leaves them to the general kernels
+    int resident = 1;
+    // nodes a CTA of it takes at most before another CTA is added, for a
+    // single solve and for a batch's members; SVX_RESIDENT_NODES and
+    // SVX_RESIDENT_BATCH_NODES (multiples of 32 up to 512, measurements)
+    int resident_nodes_single = 128;
+    int resident_nodes_batch = 512;
+    // low-priority streams of a batch's size classes, created when needed
+    std::vector<cudaStream_t> class_streams;
+    std::vector<cudaEvent_t> class_events;
     // 1: the graph form's FP32 SpMV runs on the quad copy of the operator,
     // 0: on the node-block layout; SVX_FP32_QUADS (measurements)
     int fp32_quads = 1;
@@ -274,6 +285,10 @@ struct svx_op {
     svx::DBuf<int32_t> conn;
     svx::DBuf<double> youngs, poisson;
     svx::DBuf<double> thick_elem;  // per-element thickness (batched models), else empty
+    // the chip-resident PCG's node order (svx_resident.cu): per member, slot
+    // -> node and node -> slot; built by the first solve that needs it
+    svx::DBuf<uint16_t> slot_node, node_slot;
+    int64_t slot_span = -1;  // single models: its largest slot difference (-1: not built)
     svx::Pattern pat;
     // assembled system
     svx::DBuf<double> vals;        // K after Dirichlet (the PCG operator)
@@ -406,6 +421,27 @@ struct BatchStats {
 // FP32 difference-form copy of the operator for the mixed forms (svx_pcg.cu).
 void build_fp32_operator(svx_ctx* ctx, svx_op* op);
 const double* transposed_values(svx_ctx* ctx, svx_op* op);
+// Chip-resident PCG of plane models (svx_resident.cu).
+constexpr int64_t RESIDENT_MAX_NODES = 8192;
+constexpr size_t RESIDENT_SMEM = 216 * 1024;  // of 227 KB, less the kernel's static arrays
+constexpr int RESIDENT_MAX_DEG = 9;           // neighbour blocks a thread's registers hold
+// iterations one launch may be asked for (a few seconds of work)
+constexpr int64_t RESIDENT_MAX_ITER = int64_t(1) << 22;
+constexpr int RESIDENT_STALLED = -1;  // status: a wait between CTAs ran out
+struct ResidentShape {
+    int ctas = 0, threads = 0, window = 0;
+    size_t smem = 0;
+};
+void resident_order(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_t>& node_off,
+                    std::vector<int64_t>& span);
+bool resident_shape(const svx_ctx* ctx, int64_t n, int64_t span, bool single,
+                    ResidentShape* out);
+// `count` members of op, one cluster each; all pointers on the device.
+void resident_pcg(svx_ctx* ctx, const svx_op* op, const ResidentShape& shape, bool single, cudaStream_t st,
+                  int count, const int32_t* order, const int64_t* node_off, const double* tol,
+                  const int64_t* max_iter, int64_t* out_it, double* out_res,
+                  int32_t* out_status, double* u);
+
 void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& node_off,
                const std::vector<double>& tol, const std::vector<int64_t>& max_iter,
                std::vector<int64_t>& it, std::vector<double>& res, std::vector<int32_t>& status,

@@ -2867,11 +2867,55 @@ int choose_spmv_group(const svx_op* op) {
     return pick_group(mean);
 }
 
+static const char* const RESIDENT_STALL_TEXT =
+    "resident PCG: a wait between the CTAs of a cluster ran out";
+
+// One plane model on the chip-resident cluster kernel (svx_resident.cu).
+static PcgResult pcg_resident(svx_ctx* ctx, svx_op* op, const ResidentShape& shape, double tol,
+                              long long max_iter, double* u_dev) {
+    struct Slot {
+        int64_t off[2], max_iter, it;
+        double tol, res;
+        int32_t status, pad;
+    };
+    static_assert(sizeof(Slot) <= 256, "the context's pinned scalar slot holds 256 bytes");
+    cudaStream_t st = ctx->stream;
+    DBuf<Slot> d;
+    d.alloc(ctx->pool, 1);
+    Slot* h = static_cast<Slot*>(ctx->h_scalars);
+    *h = Slot{{0, op->n_nodes}, max_iter, 0, tol, 0.0, PCG_RUNNING, 0};
+    SVX_CUDA(cudaMemcpyAsync(d.p, h, sizeof(Slot), cudaMemcpyHostToDevice, st));
+    SVX_CUDA(cudaEventRecord(ctx->ev[0], st));
+    resident_pcg(ctx, op, shape, true, st, 1, nullptr, d.p->off, &d.p->tol, &d.p->max_iter, &d.p->it,
+                 &d.p->res, &d.p->status, u_dev);
+    SVX_CUDA(cudaEventRecord(ctx->ev[1], st));
+    SVX_CUDA(cudaMemcpyAsync(h, d.p, sizeof(Slot), cudaMemcpyDeviceToHost, st));
+    SVX_CUDA(cudaStreamSynchronize(st));
+    float ms = 0.f;
+    SVX_CUDA(cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]));
+    if (h->status == RESIDENT_STALLED) throw ModelFail{SVX_CUDA_ERROR, 0, -1, RESIDENT_STALL_TEXT};
+    return PcgResult{h->status, h->it, h->res, ms};
+}
+
 PcgResult pcg_fp64(svx_ctx* ctx, svx_op* op, double tol, long long max_iter, int check_every,
                    double* u_dev) {
     const int64_t n = op->n;
     cudaStream_t st = ctx->stream;
     PcgResult out{PCG_CONVERGED, 0, 0.0, 0.0};
+    // plane models that fit on the chip; a budget so large that one launch
+    // could run for many seconds keeps the chunked launches below
+    if (op->ndof == 2 && op->n_nodes < RESIDENT_MAX_NODES && ctx->resident && ctx->pcg_smem &&
+        op->pat.max_deg <= RESIDENT_MAX_DEG && max_iter <= RESIDENT_MAX_ITER &&
+        !use_graph_form(ctx, op)) {
+        if (op->slot_span < 0) {
+            std::vector<int64_t> span{0};
+            resident_order(ctx, op, true, {0, op->n_nodes}, span);
+            op->slot_span = span[0];
+        }
+        ResidentShape shape;
+        if (resident_shape(ctx, op->n_nodes, op->slot_span, true, &shape))
+            return pcg_resident(ctx, op, shape, tol, max_iter, u_dev);
+    }
     if (check_every <= 0) check_every = auto_check_every(n, op->pat.nnz);
     DBuf<double> r, p, p2, q, partials;
     DBuf<PcgScalars> s;
@@ -3655,6 +3699,22 @@ std::vector<BatchConfig> batch_candidates(int ndof) {
 
 }  // namespace
 
+// Largest node degree of each member, one CTA per member.
+static __global__ void member_degree_kernel(const int64_t* __restrict__ node_off,
+                                            const int64_t* __restrict__ adj_ptr,
+                                            int64_t* __restrict__ out) {
+    __shared__ int top;
+    if (threadIdx.x == 0) top = 0;
+    __syncthreads();
+    int d = 0;
+    for (int64_t i = node_off[blockIdx.x] + threadIdx.x; i < node_off[blockIdx.x + 1];
+         i += blockDim.x)
+        d = max(d, int(adj_ptr[i + 1] - adj_ptr[i]));
+    atomicMax(&top, d);
+    __syncthreads();
+    if (threadIdx.x == 0) out[blockIdx.x] = top;
+}
+
 void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& node_off,
                const std::vector<double>& tol, const std::vector<int64_t>& max_iter,
                std::vector<int64_t>& it, std::vector<double>& res, std::vector<int32_t>& status,
@@ -3671,12 +3731,50 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
     auto rows_of = [&](int k) { return (node_off[k + 1] - node_off[k]) * op->ndof; };
     std::stable_sort(order.begin(), order.end(),
                      [&](int a, int b) { return rows_of(a) > rows_of(b); });
+    // FP64 plane members that fit on the chip run the resident cluster kernel,
+    // one launch per cluster shape
+    std::vector<ResidentShape> shapes(op->ndof == 2 && !mixed && ctx->resident ? count : 0);
+    if (!shapes.empty()) {
+        std::vector<int64_t> degree, span(count, 0);
+        resident_order(ctx, op, false, node_off, span);
+        if (P.max_deg > RESIDENT_MAX_DEG) {  // some member is out: find which
+            DBuf<int64_t> off, top;
+            off.alloc(ctx->pool, count + 1);
+            top.alloc(ctx->pool, count + 1);
+            degree.resize(count);
+            SVX_CUDA(cudaMemcpyAsync(off.p, node_off.data(), (count + 1) * sizeof(int64_t),
+                                     cudaMemcpyHostToDevice, st));
+            member_degree_kernel<<<count, 256, 0, st>>>(off.p, P.adj_ptr.p, top.p);
+            SVX_LAUNCH_CHECK();
+            SVX_CUDA(cudaMemcpyAsync(degree.data(), top.p, count * sizeof(int64_t),
+                                     cudaMemcpyDeviceToHost, st));
+            SVX_CUDA(cudaStreamSynchronize(st));
+        }
+        for (int k = 0; k < count; ++k) {
+            if (max_iter[k] > RESIDENT_MAX_ITER ||
+                (!degree.empty() && degree[k] > RESIDENT_MAX_DEG) ||
+                !resident_shape(ctx, node_off[k + 1] - node_off[k], span[k], false, &shapes[k]))
+                shapes[k] = ResidentShape{};
+        }
+    }
+    auto resident = [&](int k) { return !shapes.empty() && shapes[k].ctas > 0; };
+    const auto general_end = std::stable_partition(order.begin(), order.end(),
+                                                   [&](int k) { return !resident(k); });
+    const int n_general = int(general_end - order.begin());
+    // resident members by shape, the largest shapes first, then by size
+    std::stable_sort(general_end, order.end(), [&](int x, int y) {
+        const ResidentShape &a = shapes[x], &b = shapes[y];
+        return a.ctas * a.threads != b.ctas * b.threads ? a.ctas * a.threads > b.ctas * b.threads
+                                                        : a.threads > b.threads;
+    });
     int n_large = 0;
-    while (n_large < count && rows_of(order[n_large]) >= cluster_min_dof(op->ndof)) ++n_large;
-    const int n_small = count - n_large;
-    // small class first in the order array, then the large class
-    std::vector<int32_t> ordered(order.begin() + n_large, order.end());
+    while (n_large < n_general && rows_of(order[n_large]) >= cluster_min_dof(op->ndof)) ++n_large;
+    const int n_small = n_general - n_large;
+    // small class first in the order array, then the large class, then the
+    // resident members
+    std::vector<int32_t> ordered(order.begin() + n_large, order.begin() + n_general);
     ordered.insert(ordered.end(), order.begin(), order.begin() + n_large);
+    ordered.insert(ordered.end(), order.begin() + n_general, order.end());
     DBuf<int32_t> d_order, d_status;
     DBuf<int64_t> d_off, d_maxit, d_it, d_cap;
     DBuf<double> d_tol, d_res, r, p, q, d_hi, d_lo;
@@ -3777,6 +3875,37 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
                              mixed ? d_fp32.p : nullptr, u_sv, r_sv, p_sv);
         SVX_CUDA(cudaEventRecord(ctx->join_ev, ctx->aux_stream));
     }
+    int n_class = 0;
+    for (int k0 = n_general; k0 < count; ++n_class) {
+        // the run of members of one shape, its window the largest of them
+        ResidentShape shape = shapes[ordered[k0]];
+        int k1 = k0 + 1;
+        for (; k1 < count && shapes[ordered[k1]].ctas == shape.ctas &&
+               shapes[ordered[k1]].threads == shape.threads;
+             ++k1) {
+            shape.window = std::max(shape.window, shapes[ordered[k1]].window);
+            shape.smem = std::max(shape.smem, shapes[ordered[k1]].smem);
+        }
+        if (int(ctx->class_streams.size()) <= n_class) {
+            int least = 0, greatest = 0;
+            SVX_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+            cudaStream_t cs = nullptr;
+            cudaEvent_t ce = nullptr;
+            SVX_CUDA(cudaStreamCreateWithPriority(&cs, cudaStreamNonBlocking, least));
+            ctx->class_streams.push_back(cs);
+            SVX_CUDA(cudaEventCreateWithFlags(&ce, cudaEventDisableTiming));
+            ctx->class_events.push_back(ce);
+        }
+        if (n_class == 0) SVX_CUDA(cudaEventRecord(ctx->fork_ev, pst));
+        cudaStream_t cs = ctx->class_streams[n_class];
+        SVX_CUDA(cudaStreamWaitEvent(cs, ctx->fork_ev, 0));
+        resident_pcg(ctx, op, shape, false, cs, k1 - k0, d_order.p + k0, d_off.p, d_tol.p, d_maxit.p,
+                     d_it.p, d_res.p, d_status.p, op->u.p);
+        SVX_CUDA(cudaEventRecord(ctx->class_events[n_class], cs));
+        k0 = k1;
+    }
+    for (int c = 0; c < n_class; ++c)
+        SVX_CUDA(cudaStreamWaitEvent(pst, ctx->class_events[c], 0));
     if (n_small > 0) launch(choice, d_maxit.p, n_small);
     if (n_large > 0) SVX_CUDA(cudaStreamWaitEvent(pst, ctx->join_ev, 0));
     SVX_CUDA(cudaEventRecord(ctx->ev[1], pst));
@@ -3813,14 +3942,19 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
     SVX_CUDA(cudaStreamSynchronize(st));
     float ms = 0.f;
     SVX_CUDA(cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]));
+    for (int k = 0; k < count; ++k)
+        if (status[k] == RESIDENT_STALLED)
+            throw ModelFail{SVX_CUDA_ERROR, 0, -1, RESIDENT_STALL_TEXT};
     for (int k = 0; k < count; ++k) cond[k] = hi[k] / lo[k];
     op->has_solution = true;
     if (stats) {
         stats->fp32_iterations = 0;
         for (int64_t v : f32) stats->fp32_iterations += v;
         stats->ms_solve = ms;
-        stats->threads_per_cta = cfg.bs;
-        stats->lanes_per_node = cfg.g;
+        // the shape of most members: the resident kernel's, or the autotuned one
+        const bool res = count - n_general > n_small;
+        stats->threads_per_cta = res ? ctx->resident_nodes_batch : cfg.bs;
+        stats->lanes_per_node = res ? 1 : cfg.g;
         stats->cluster_members = n_large;
         stats->member_nnz = std::move(nnz);
     }
