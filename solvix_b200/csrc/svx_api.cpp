@@ -470,7 +470,11 @@ svx_op* assemble_impl(svx_ctx* ctx, const svx_flat_model_t* m, uint32_t flags,
     upload(ctx, op->poisson, m->poisson, size_t(op->n_elem));
     if (thick_elem) upload(ctx, op->thick_elem, thick_elem, size_t(op->n_elem));
     int max_nn = 0;
-    for (int64_t e = 0; e < op->n_elem; ++e) max_nn = std::max(max_nn, node_count(m->kind[e]));
+    op->all_hex = op->n_elem > 0;
+    for (int64_t e = 0; e < op->n_elem; ++e) {
+        max_nn = std::max(max_nn, node_count(m->kind[e]));
+        op->all_hex = op->all_hex && m->kind[e] == SVX_C3D8;
+    }
     op->pat.max_nn = std::max(max_nn, 1);
     const int max_N = max_nn * m->ndof;
     op->pat.ke_stride = std::max(1, max_N * max_N);
@@ -860,7 +864,7 @@ void run_batch(svx_ctx* ctx, int32_t count, const svx_flat_model_t* const* model
         std::vector<double> res, cond;
         std::vector<int32_t> status;
         BatchStats bs;
-        batch_pcg(ctx, op.get(), L, node_off, tol, mi, it, res, status, cond, &bs,
+        batch_pcg(ctx, op.get(), L, node_off, elem_off, tol, mi, it, res, status, cond, &bs,
                   o.precision == SVX_MIXED);
         run.wall_solve += since(t_phase);
         t_phase = clock::now();
@@ -967,6 +971,14 @@ int svx_ctx_create(int device, svx_ctx_t** out) {
         if (const char* e = std::getenv("SVX_PCG_STAGE")) ctx->pcg_stage = (e[0] != '0');
         if (const char* e = std::getenv("SVX_FP32_QUADS")) ctx->fp32_quads = (e[0] != '0');
         if (const char* e = std::getenv("SVX_RESIDENT")) ctx->resident = (e[0] != '0');
+        if (const char* e = std::getenv("SVX_HEX")) ctx->hex = (e[0] != '0');
+        if (const char* e = std::getenv("SVX_BRICK_MAX_ELEMS"))
+            ctx->brick_max_elems = std::min(std::atoi(e), BRICK_MAX_ELEMS);
+        if (const char* e = std::getenv("SVX_BRICK_ELEMS")) ctx->brick_elems = std::atoi(e);
+        if (const char* e = std::getenv("SVX_BRICK_BATCH_ELEMS"))
+            ctx->brick_batch_elems = std::atoi(e);
+        if (const char* e = std::getenv("SVX_HEX_MIN_NODES"))
+            ctx->hex_min_nodes = std::strtoll(e, nullptr, 10);
         auto nodes_env = [](const char* name, int& to) {
             const char* e = std::getenv(name);
             const int v = e ? std::atoi(e) : 0;

@@ -207,6 +207,17 @@ struct svx_ctx {
     // SVX_RESIDENT_BATCH_NODES (multiples of 32 up to 512, measurements)
     int resident_nodes_single = 128;
     int resident_nodes_batch = 512;
+    // 1: FP64 solves of all-C3D8 models of at least hex_min_nodes nodes apply
+    // the operator element by element (svx_hex.cu, svx_brick.cu); SVX_HEX=0,
+    // SVX_HEX_MIN_NODES and SVX_BRICK_MAX_ELEMS (measurements)
+    int hex = 1;
+    long long hex_min_nodes = 14000, hex_batch_min_nodes = 2048;
+    int brick_max_elems = 288;  // of a single model's brick; above: the graph form
+    // elements of a brick at least, for a single model, and at most for a
+    // batch's members before another CTA is added; SVX_BRICK_ELEMS and
+    // SVX_BRICK_BATCH_ELEMS (measurements)
+    int brick_elems = 128;
+    int brick_batch_elems = 512;
     // low-priority streams of a batch's size classes, created when needed
     std::vector<cudaStream_t> class_streams;
     std::vector<cudaEvent_t> class_events;
@@ -270,6 +281,44 @@ struct Pattern {
     DBuf<int32_t> diag_pos;    // [n] nnz index of the diagonal
 };
 
+// What the element-by-element operator of a C3D8 model keeps (svx_hex.cu).
+struct HexOperator {
+    DBuf<double> rdet;    // [8][n_elem] 1 / det of the eightfold Jacobian
+    DBuf<double2> lame;   // [n_elem] Lame constants / 512
+    DBuf<double> x4;      // [n_nodes][4] coordinates
+    DBuf<uint32_t> slot;  // [max_slots][n_nodes] force offsets of a node's slots
+};
+
+// The bricks of C3D8 models (svx_brick.cu).
+struct BrickView {
+    int bricks, ncap;              // ncap: nodes a brick may have
+    int held, lists;               // elements and chunk nodes held in shared memory
+    const int32_t *elem0, *elem1;  // [bricks] its elements, positions in `order`
+    const int32_t* member;         // [bricks]
+    const int32_t* chunk0;         // [bricks] its first chunk
+    const int32_t* order;          // [n_elem] elements by layer
+    int32_t* count;                // [bricks] nodes
+    int32_t* node;                 // [bricks][ncap]
+    uint16_t* lconn;               // [n_elem][8] nodes of the brick, in `order`
+    uint32_t* entry;               // [n_nodes][8] brick * ncap + place, ascending (~0: none)
+    // per chunk: its nodes (places in the brick), and eight offsets of staged
+    // forces for each, in ascending element order
+    uint16_t *cnode, *ref;
+    int32_t* ccount;
+};
+struct BrickOperator {
+    int bricks = 0, ncap = 0, held = 0, lists = 0;
+    int state = 0;     // single models: 0 not built, 1 built, -1 does not fit
+    DBuf<int32_t> elem0, elem1, member, chunk0, order, count, node, ccount, member_brick;
+    DBuf<uint16_t> lconn, cnode, ref;
+    DBuf<uint32_t> entry;
+    DBuf<double> geo;
+    BrickView view() const {
+        return BrickView{bricks,  ncap,   held,    lists,   elem0.p, elem1.p, member.p, chunk0.p,
+                         order.p, count.p, node.p, lconn.p, entry.p, cnode.p, ref.p,    ccount.p};
+    }
+};
+
 }  // namespace svx
 
 // ------------------------------------------------------------------ operator
@@ -290,6 +339,9 @@ struct svx_op {
     svx::DBuf<uint16_t> slot_node, node_slot;
     int64_t slot_span = -1;  // single models: its largest slot difference (-1: not built)
     svx::Pattern pat;
+    bool all_hex = false;  // every element is a C3D8
+    svx::HexOperator hex;  // built by the first solve that applies it
+    svx::BrickOperator brick;
     // assembled system
     svx::DBuf<double> vals;        // K after Dirichlet (the PCG operator)
     // K again with each node's values ordered (da, db, neighbour slot), the
@@ -421,6 +473,37 @@ struct BatchStats {
 // FP32 difference-form copy of the operator for the mixed forms (svx_pcg.cu).
 void build_fp32_operator(svx_ctx* ctx, svx_op* op);
 const double* transposed_values(svx_ctx* ctx, svx_op* op);
+// Element-by-element FP64 operator of C3D8 models (svx_hex.cu).
+struct HexWork {
+    DBuf<double> fe, p4, partials;
+    void alloc(svx_ctx* ctx, const svx_op* op);
+};
+bool hex_applies(const svx_ctx* ctx, const svx_op* op);
+void hex_prepare(svx_ctx* ctx, svx_op* op);
+// p in rows of four, before the first iteration on a direction p.
+void hex_start(const svx_op* op, HexWork& w, cudaStream_t st, const double* p);
+// One iteration of the graph form (three launches, PcgScalars' rules).
+void hex_iteration(const svx_op* op, HexWork& w, cudaStream_t st, const double* inv_diag,
+                   double* u, double* r, double* p, PcgScalars* s);
+
+// Jacobi-PCG of C3D8 models on bricks of elements (svx_brick.cu).
+constexpr int BRICK_LAYERS = 1024;
+constexpr int BRICK_MAX_ELEMS = 2016;        // seven chunks; 16,384 references
+constexpr size_t BRICK_SMEM = 226 * 1024;    // of 227 KB, less the kernel's static arrays
+struct BrickWork {
+    DBuf<double> exchange, slots, vec;
+    DBuf<GridBarrier> gb;
+    void alloc(svx_ctx* ctx, const svx_op* op, bool single);
+};
+void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_t>& node_off,
+                 const std::vector<int64_t>& elem_off, std::vector<int>& nbricks);
+void brick_grid_launch(svx_ctx* ctx, const svx_op* op, BrickWork& w, double* u, double* r,
+                       double* p, PcgScalars* s, int chunk);
+void brick_batch_launch(const svx_op* op, BrickWork& w, cudaStream_t st, int ctas, int count,
+                        const int32_t* order, double* u, const double* tol,
+                        const int64_t* max_iter, int64_t* out_it, double* out_res,
+                        int32_t* out_status);
+
 // Chip-resident PCG of plane models (svx_resident.cu).
 constexpr int64_t RESIDENT_MAX_NODES = 8192;
 constexpr size_t RESIDENT_SMEM = 216 * 1024;  // of 227 KB, less the kernel's static arrays
@@ -443,6 +526,7 @@ void resident_pcg(svx_ctx* ctx, const svx_op* op, const ResidentShape& shape, bo
                   int32_t* out_status, double* u);
 
 void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& node_off,
+               const std::vector<int64_t>& elem_off,
                const std::vector<double>& tol, const std::vector<int64_t>& max_iter,
                std::vector<int64_t>& it, std::vector<double>& res, std::vector<int32_t>& status,
                std::vector<double>& cond, BatchStats* stats, bool mixed = false);

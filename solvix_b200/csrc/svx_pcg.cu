@@ -2371,8 +2371,16 @@ struct PcgRun {
     double* partials;
     PcgScalars* s;
     PcgScalars* h_s;  // pinned
+    HexWork* hex = nullptr;  // FP64 C3D8: K applied element by element
+    BrickWork* brick = nullptr;  // FP64 C3D8: the persistent form on bricks
 
     void enqueue_iteration(cudaStream_t st) {
+        if constexpr (std::is_same<M, double>::value) {
+            if (hex) {
+                hex_iteration(op, *hex, st, inv_diag, u, r, p, s);
+                return;
+            }
+        }
         if constexpr (std::is_same<M, float>::value) {
             if (vals == op->vals32.p && op->vals32q.p)
                 launch_spmv_fp32(op, G, grid_r, st, p, q, partials, s);
@@ -2621,9 +2629,46 @@ struct PcgRun {
         }
     }
 
+    // The persistent form on bricks of elements (svx_brick.cu): cooperative
+    // launches of up to `chunk` iterations each.
+    int iterate_brick(int chunk) {
+        if constexpr (std::is_same<M, double>::value && std::is_same<V, double>::value &&
+                      std::is_same<U, double>::value) {
+            cudaStream_t st = ctx->stream;
+            SVX_CUDA(cudaMemcpyAsync(h_s, s, sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
+            SVX_CUDA(cudaStreamSynchronize(st));
+            const long long launches_max = h_s->max_iter / chunk + 2;
+            int status = h_s->status;
+            GridBarrier hgb{};
+            for (long long launch = 0; status == PCG_RUNNING; ++launch) {
+                if (launch >= launches_max)
+                    throw ModelFail{SVX_CUDA_ERROR, 0, -1,
+                                    "PCG status did not leave RUNNING within max_iter"};
+                brick_grid_launch(ctx, op, *brick, u, r, p, s, chunk);
+                SVX_CUDA(cudaMemcpyAsync(h_s, s, sizeof(PcgScalars), cudaMemcpyDeviceToHost,
+                                         st));
+                SVX_CUDA(cudaMemcpyAsync(&hgb, brick->gb.p, sizeof(GridBarrier),
+                                         cudaMemcpyDeviceToHost, st));
+                SVX_CUDA(cudaStreamSynchronize(st));
+                if (hgb.error)
+                    throw ModelFail{SVX_CUDA_ERROR, 0, -1,
+                                    "persistent PCG: a grid barrier wait ran out (blocks not "
+                                    "co-resident)"};
+                status = h_s->status;
+            }
+            return status;
+        } else {
+            (void)chunk;
+            return -1;
+        }
+    }
+
     // Runs until the device status leaves RUNNING; returns the status.
     int iterate(int check_every) {
         cudaStream_t st = ctx->stream;
+        if constexpr (std::is_same<M, double>::value && std::is_same<V, double>::value) {
+            if (hex) hex_start(op, *hex, st, p);
+        }
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
         SVX_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -2897,6 +2942,35 @@ static PcgResult pcg_resident(svx_ctx* ctx, svx_op* op, const ResidentShape& sha
     return PcgResult{h->status, h->it, h->res, ms};
 }
 
+// Gives an FP64 run of a C3D8 model its element-by-element form, where it
+// has one: bricks while a model's bricks fit the chip, the graph form above.
+static void wire_hex(svx_ctx* ctx, svx_op* op, PcgRun<double, double, double>& run, HexWork& hex,
+                     BrickWork& brick) {
+    if (!hex_applies(ctx, op)) return;
+    if (!(ctx->graph_min_nnz >= 0 && use_graph_form(ctx, op)) && op->brick.state == 0) {
+        int coop = 0;
+        SVX_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
+        const int64_t per = std::max<int64_t>(ctx->brick_elems,
+                                              (op->n_elem + ctx->sm_count - 1) / ctx->sm_count);
+        std::vector<int> nbricks{coop && per <= ctx->brick_max_elems
+                                     ? int((op->n_elem + per - 1) / per) : 0};
+        if (nbricks[0] > 0) brick_build(ctx, op, true, {0, op->n_nodes}, {0, op->n_elem}, nbricks);
+        op->brick.state = nbricks[0] > 0 ? 1 : -1;
+    }
+    if (op->brick.state > 0) {
+        brick.alloc(ctx, op, true);
+        run.brick = &brick;
+        return;
+    }
+    // a model that the shared-memory kernel holds and that has no bricks keeps
+    // its assembled K: a 35^3 cube runs 19.7 us an iteration on it and 22.4 in
+    // the graph form's three launches; at 180 x 16 x 16 it is 24.0 and 22.2
+    if (!use_graph_form(ctx, op) && op->n_elem < 45000 && ctx->brick_max_elems > 1) return;
+    hex_prepare(ctx, op);
+    hex.alloc(ctx, op);
+    run.hex = &hex;
+}
+
 PcgResult pcg_fp64(svx_ctx* ctx, svx_op* op, double tol, long long max_iter, int check_every,
                    double* u_dev) {
     const int64_t n = op->n;
@@ -2958,10 +3032,17 @@ PcgResult pcg_fp64(svx_ctx* ctx, svx_op* op, double tol, long long max_iter, int
     run.partials = partials.p;
     run.s = s.p;
     run.h_s = hs.h;
+    HexWork hex;
+    BrickWork brick;
+    wire_hex(ctx, op, run, hex, brick);
     SVX_CUDA(cudaMemcpyAsync(hs.h, s.p, sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
     SVX_CUDA(cudaStreamSynchronize(st));
     int status = hs.h->status;
-    if (status == PCG_RUNNING) {
+    if (status == PCG_RUNNING && run.brick) {
+        status = run.iterate_brick(persistent_chunk(op->pat.nnz));
+    } else if (status == PCG_RUNNING && run.hex) {
+        status = run.iterate(check_every);
+    } else if (status == PCG_RUNNING) {
         // the graph form starts from the init kernel's p = z0 too: a
         // persistent launch that cannot start leaves p untouched
         status = -1;
@@ -3079,6 +3160,9 @@ PcgResult pcg_mixed(svx_ctx* ctx, svx_op* op, double tol, long long max_iter, do
     wire(exact);
     sloppy.vals = op->vals32.p;
     exact.vals = op->vals.p;
+    HexWork hex;
+    BrickWork brick;
+    wire_hex(ctx, op, exact, hex, brick);
 
     auto true_residual = [&]() -> double {
         const Pattern& P = op->pat;
@@ -3117,7 +3201,9 @@ PcgResult pcg_mixed(svx_ctx* ctx, svx_op* op, double tol, long long max_iter, do
     double res = hs.h->res;
     const int chunk = persistent_chunk(op->pat.nnz);
     auto run = [&](auto& pcg) -> int {
-        const int stt = graph ? pcg.iterate(check_every) : pcg.iterate_persistent(chunk);
+        const int stt = pcg.brick            ? pcg.iterate_brick(chunk)
+                        : graph || pcg.hex ? pcg.iterate(check_every)
+                                           : pcg.iterate_persistent(chunk);
         if (stt < 0)
             throw ModelFail{SVX_CUDA_ERROR, 0, -1,
                             "mixed precision below 50M nonzeros needs a cooperative launch"};
@@ -3716,7 +3802,7 @@ static __global__ void member_degree_kernel(const int64_t* __restrict__ node_off
 }
 
 void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& node_off,
-               const std::vector<double>& tol, const std::vector<int64_t>& max_iter,
+               const std::vector<int64_t>& elem_off, const std::vector<double>& tol, const std::vector<int64_t>& max_iter,
                std::vector<int64_t>& it, std::vector<double>& res, std::vector<int32_t>& status,
                std::vector<double>& cond, BatchStats* stats, bool mixed) {
     cudaStream_t st = ctx->stream;
@@ -3757,6 +3843,28 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
                 shapes[k] = ResidentShape{};
         }
     }
+    // FP64 C3D8 members on bricks, a cluster of 1, 2, 4, 8 or 16 CTAs each
+    std::vector<int> nbricks;
+    if (op->ndof == 3 && !mixed && ctx->hex && op->all_hex) {
+        nbricks.assign(count, 0);
+        bool any = false;
+        for (int k = 0; k < count; ++k) {
+            const int64_t ne = elem_off[k + 1] - elem_off[k];
+            if (node_off[k + 1] - node_off[k] < ctx->hex_batch_min_nodes ||
+                ne > 16 * int64_t(BRICK_MAX_ELEMS))
+                continue;
+            int c = 1;
+            while (c < 16 && int64_t(c) * ctx->brick_batch_elems < ne) c *= 2;
+            nbricks[k] = c;
+            any = true;
+        }
+        if (any) brick_build(ctx, op, false, node_off, elem_off, nbricks);
+        for (int k = 0; any && k < count; ++k)
+            if (nbricks[k]) {
+                shapes.resize(count);
+                shapes[k].ctas = nbricks[k];
+            }
+    }
     auto resident = [&](int k) { return !shapes.empty() && shapes[k].ctas > 0; };
     const auto general_end = std::stable_partition(order.begin(), order.end(),
                                                    [&](int k) { return !resident(k); });
@@ -3764,6 +3872,7 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
     // resident members by shape, the largest shapes first, then by size
     std::stable_sort(general_end, order.end(), [&](int x, int y) {
         const ResidentShape &a = shapes[x], &b = shapes[y];
+        if (op->ndof == 3) return a.ctas > b.ctas;
         return a.ctas * a.threads != b.ctas * b.threads ? a.ctas * a.threads > b.ctas * b.threads
                                                         : a.threads > b.threads;
     });
@@ -3876,6 +3985,11 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
         SVX_CUDA(cudaEventRecord(ctx->join_ev, ctx->aux_stream));
     }
     int n_class = 0;
+    BrickWork brick;
+    if (op->ndof == 3 && n_general < count) {
+        brick.alloc(ctx, op, false);
+        SVX_CUDA(cudaMemsetAsync(brick.slots.p, 0, brick.slots.bytes(), pst));
+    }
     for (int k0 = n_general; k0 < count; ++n_class) {
         // the run of members of one shape, its window the largest of them
         ResidentShape shape = shapes[ordered[k0]];
@@ -3899,8 +4013,12 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
         if (n_class == 0) SVX_CUDA(cudaEventRecord(ctx->fork_ev, pst));
         cudaStream_t cs = ctx->class_streams[n_class];
         SVX_CUDA(cudaStreamWaitEvent(cs, ctx->fork_ev, 0));
-        resident_pcg(ctx, op, shape, false, cs, k1 - k0, d_order.p + k0, d_off.p, d_tol.p, d_maxit.p,
-                     d_it.p, d_res.p, d_status.p, op->u.p);
+        if (op->ndof == 3)
+            brick_batch_launch(op, brick, cs, shape.ctas, k1 - k0, d_order.p + k0, op->u.p,
+                               d_tol.p, d_maxit.p, d_it.p, d_res.p, d_status.p);
+        else
+            resident_pcg(ctx, op, shape, false, cs, k1 - k0, d_order.p + k0, d_off.p, d_tol.p,
+                         d_maxit.p, d_it.p, d_res.p, d_status.p, op->u.p);
         SVX_CUDA(cudaEventRecord(ctx->class_events[n_class], cs));
         k0 = k1;
     }
@@ -3953,9 +4071,10 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
         stats->ms_solve = ms;
         // the shape of most members: the resident kernel's, or the autotuned one
         const bool res = count - n_general > n_small;
-        stats->threads_per_cta = res ? ctx->resident_nodes_batch : cfg.bs;
+        stats->threads_per_cta = !res ? cfg.bs : op->ndof == 3 ? 256 : ctx->resident_nodes_batch;
         stats->lanes_per_node = res ? 1 : cfg.g;
-        stats->cluster_members = n_large;
+        // the documented classes: 3D >= 4,096 rows, 2D >= 16,384
+        stats->cluster_members = n_large + (op->ndof == 3 ? count - n_general : 0);
         stats->member_nnz = std::move(nnz);
     }
 }

@@ -41,6 +41,7 @@
 // largest members ran alone at the end).
 
 #include "svx_internal.h"
+#include "svx_warp.h"
 
 #include <cmath>
 #include <cstddef>
@@ -133,34 +134,6 @@ __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-}
-
-// D = A B with 8 x 4 by 4 x 8 FP64 operands: the lane's A element is (lane /
-// 4, lane % 4), its B element (lane % 4, lane / 4), its two D elements
-// (lane / 4, 2 (lane % 4) + {0, 1}).
-__device__ __forceinline__ void mma(double& d0, double& d1, double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%4,%4};"
-                 : "=d"(d0), "=d"(d1) : "d"(a), "d"(b), "d"(0.0));
-}
-// Sum over the warp, the same bits in every lane: ones x V gives the lane
-// the sums of two quads of lanes, which add up to a quarter of the total
-// per lane % 4; quarters x ones gives the total.
-__device__ __forceinline__ double quarter_sum(double v) {
-    double a, b;
-    mma(a, b, 1.0, v);
-    return a + b;
-}
-__device__ __forceinline__ double lane_sum(double v) {
-    double a, b;
-    mma(a, b, quarter_sum(v), 1.0);
-    return a;
-}
-// Two sums at once: lanes 0-15 get x's, lanes 16-31 get y's.
-__device__ __forceinline__ double lane_sum_pair(double x, double y, int lane) {
-    const double qx = quarter_sum(x), qy = quarter_sum(y);
-    double a, b;
-    mma(a, b, lane < 16 ? qx : qy, 1.0);
-    return a;
 }
 
 // x / y from y's reciprocal: one residual correction brings the product to
