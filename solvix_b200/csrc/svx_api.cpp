@@ -412,6 +412,7 @@ void device_assemble(svx_ctx* ctx, svx_op* op) {
     op->vals32.reset();
     op->vals32q.reset();
     op->valsT.reset();
+    op->vals32T.reset();
     apply_dirichlet(ctx, op);
     op->spmv_group = choose_spmv_group(op);
     SVX_CUDA(cudaEventRecord(ctx->ev[3], st));

@@ -10,12 +10,8 @@
 // that several of them touch, each one's partial force.  Every brick then
 // adds the partials in the same order and updates r, u, z and p of all its
 // nodes itself, so the copies of a shared node stay bitwise equal and p is
-// never sent: two exchanges an iteration, one for p.Kp (the sum of the
-// elements' p_e.f_e) and the partial forces, one for r.r and r.z.  An
-// exchange is no barrier: every CTA posts its sum with the exchange's number
-// in one 128-bit word and reads the others' words until they carry that
-// number (bounded).  A counting barrier and the partial sums behind it took
-// 4,000 + 3,800 cycles for 148 CTAs.
+// never sent: two barriers an iteration, one for p.Kp (the sum of the
+// elements' p_e.f_e) and the partial forces, one for r.r and r.z.
 //
 // Bricks are runs of elements ordered by layers along the model's longest
 // side, so a cantilever's bricks are slabs with two neighbours; any order is
@@ -23,15 +19,16 @@
 // thread; forces are staged in shared memory and each node sums its own in
 // ascending order, without atomics.
 //
-// Measured (one B200): 160 x 16 x 16 16.4 us an iteration (19.7 on the
-// assembled K from L2), 120 x 16 x 16 13.9 (16.5), 120 x 12 x 12 12.6 (13.3);
+// Measured (one B200): 160 x 16 x 16 15.5 us an iteration (19.7 on the
+// assembled K from L2), 120 x 12 x 12 10.3 (13.3), 120 x 10 x 10 9.5 (11.3);
 // below some 14,000 nodes K from L2 is as fast, above 288 elements a CTA the
 // graph form (svx_hex.cu) is.  40 members of 20..120 x 4..16^2 as one batch:
 // 99 ms of device time (224 on clusters streaming K from HBM).  An iteration
 // of the 160 x 16 x 16 model, in thousands of cycles of a CTA: forces 11.4 (a
 // full chunk of two warps a scheduler at the FP64 rate, and one of 21
 // elements), their sums 3.2, the two exchanges 12 with the wait for the
-// slowest brick, node updates 3.6.
+// slowest brick, node updates 3.6 (posting the sums as numbered 128-bit words
+// that every CTA polls, instead of the counting barrier: 16.4 us).
 //
 // GRID: one model over the whole device (cooperative launch), chunks of
 // iterations on PcgScalars' state like the other persistent
@@ -39,6 +36,7 @@
 
 #include "svx_internal.h"
 #include "svx_hex.h"
+#include "svx_grid.h"
 #include "svx_warp.h"
 
 #include <cmath>
@@ -332,42 +330,6 @@ __global__ void geometry_kernel(int64_t n_elem, const int32_t* __restrict__ orde
 }
 
 // ------------------------------------------------------------ solving
-// One CTA's contribution to a sum over a model's bricks and the exchange it
-// belongs to, read and written as one 128-bit word.
-struct __align__(16) Slot {
-    double v;
-    unsigned long long seq;
-};
-// (releases what the CTA wrote before)
-__device__ __forceinline__ void post_release(Slot* s, double v, unsigned long long seq) {
-    asm volatile(
-        "{\n .reg .b128 w;\n mov.b128 w, {%1, %2};\n"
-        " st.release.gpu.global.b128 [%0], w;\n}" ::"l"(s),
-        "l"(__double_as_longlong(v)), "l"(seq) : "memory");
-}
-__device__ __forceinline__ void post(Slot* s, double v, unsigned long long seq) {
-    asm volatile(
-        "{\n .reg .b128 w;\n mov.b128 w, {%1, %2};\n"
-        " st.relaxed.gpu.global.b128 [%0], w;\n}" ::"l"(s),
-        "l"(__double_as_longlong(v)), "l"(seq) : "memory");
-}
-template <bool ACQUIRE>
-__device__ __forceinline__ bool peek(const Slot* s, double& v, unsigned long long seq) {
-    long long x;
-    unsigned long long q;
-    if constexpr (ACQUIRE)
-        asm volatile(
-            "{\n .reg .b128 w;\n ld.acquire.gpu.global.b128 w, [%2];\n"
-            " mov.b128 {%0, %1}, w;\n}"
-            : "=l"(x), "=l"(q) : "l"(s) : "memory");
-    else
-        asm volatile(
-            "{\n .reg .b128 w;\n ld.relaxed.gpu.global.b128 w, [%2];\n"
-            " mov.b128 {%0, %1}, w;\n}"
-            : "=l"(x), "=l"(q) : "l"(s) : "memory");
-    v = __longlong_as_double(x);
-    return q == seq;
-}
 __device__ __forceinline__ void copy_async4(void* to, const void* from) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
                      unsigned(__cvta_generic_to_shared(to))), "l"(from) : "memory");
@@ -384,41 +346,6 @@ __device__ __forceinline__ void cluster_meet() {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
-constexpr int MAX_BRICKS = 160;        // of a model (bricks <= SMs)
-constexpr int POLLS = 1 << 21;         // of a slot before giving up (a second or two)
-
-// One warp: the sum of the slots of `nb` bricks, lanes over the bricks in a
-// fixed order; false when a slot does not arrive in time.  POLL = false: the
-// slots are complete (the CTAs met at a barrier).  ACQUIRE: what was released
-// with the slots is visible afterwards.
-template <bool POLL, bool ACQUIRE>
-__device__ __forceinline__ bool collect(const Slot* s, int stride, int nb,
-                                        unsigned long long seq, int lane, double& sum) {
-    constexpr int PER = MAX_BRICKS / 32;
-    double v[PER];
-    bool have[PER];
-#pragma unroll
-    for (int j = 0; j < PER; ++j) {
-        v[j] = 0.0;
-        have[j] = lane + 32 * j >= nb;
-    }
-    bool all = false;
-    for (int k = 0; k < (POLL ? POLLS : 1) && !all; ++k) {
-        all = true;
-#pragma unroll
-        for (int j = 0; j < PER; ++j)
-            if (!have[j]) have[j] = peek<ACQUIRE>(s + stride * (lane + 32 * j), v[j], seq) || !POLL;
-#pragma unroll
-        for (int j = 0; j < PER; ++j) all = all && have[j];
-    }
-    const bool ok = __all_sync(0xffffffffu, all);
-    double t = 0.0;
-#pragma unroll
-    for (int j = 0; j < PER; ++j) t += v[j];
-    sum = lane_sum(t);
-    return ok;
-}
-
 struct BrickArgs {
     BrickView b;
     int64_t n_elem;
@@ -429,7 +356,7 @@ struct BrickArgs {
     double *u, *r, *p;        // node vectors (grid: state between launches)
     double *rb, *ub, *db;     // bricks' copies of r, u, 1 / K_ii (vectors not in shared memory)
     double* rows;             // [2][bricks * ncap][4] partial forces, in turn
-    Slot* slots;              // [3][bricks] p.Kp, r.r, r.z (zero before the launch)
+    double* part;             // [3][bricks] sums of each brick: p.Kp, then r.r and r.z
     // grid
     PcgScalars* s;
     GridBarrier* gb;
@@ -452,7 +379,6 @@ __global__ void __launch_bounds__(CH, 1) brick_pcg_kernel(BrickArgs a) {
     constexpr bool SM = GRID;
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ double wa[WARPS], wb[2 * WARPS], tot[3];
-    __shared__ int arrived;
     const BrickView& b = a.b;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     int brick, brick0, nb, inst = 0;
@@ -578,42 +504,50 @@ __global__ void __launch_bounds__(CH, 1) brick_pcg_kernel(BrickArgs a) {
         fetch_lists(0, 0);
     }
     copies_done();
-    Slot* slot_a = a.slots + brick0;
-    Slot* slot_b = a.slots + b.bricks + 2 * brick0;
-    // r.r and r.z of this CTA, posted as exchange `seq`
-    auto post_b = [&](double x, double y, unsigned long long seq) {
+    unsigned target = 0;
+    auto meet = [&]() -> bool {
+        if constexpr (GRID) return grid_sync(a.gb, gridDim.x, target);
+        cluster_meet();
+        return true;
+    };
+    double* part_a = a.part + brick0;
+    double* part_b = a.part + ((b.bricks + 1) & ~1) + 2 * brick0;  // 16-byte aligned
+    // r.r and r.z of this CTA to `part_b`; the model's after the CTAs met, read
+    // by one warp (all warps of 148 CTAs reading the same few lines took 3,800
+    // cycles)
+    auto sums_b = [&](double x, double y, double& tx, double& ty) -> bool {
         const double v = lane_sum_pair(x, y, lane);
         if ((lane & 15) == 0) wb[2 * warp + (lane >> 4)] = v;
         __syncthreads();
         if (warp == 0) {
             const double w = lane_sum_pair(lane < WARPS ? wb[2 * lane] : 0.0,
                                            lane < WARPS ? wb[2 * lane + 1] : 0.0, lane);
-            if ((lane & 15) == 0)
-                post(slot_b + 2 * (brick - brick0) + (lane >> 4), w, seq);
+            if ((lane & 15) == 0) part_b[2 * (brick - brick0) + (lane >> 4)] = w;
         }
-    };
-    // their sums over the model; warps 0 and 1 read one each
-    auto total_b = [&](double& x, double& y, unsigned long long seq) -> bool {
-        if constexpr (!GRID) cluster_meet();
-        if (warp < 2) {
-            double s;
-            const bool ok = collect<GRID, false>(slot_b + warp, 2, nb, seq, lane, s);
+        if (!meet()) return false;
+        if (warp == 0) {
+            double sx = 0.0, sy = 0.0;
+            for (int k = lane; k < nb; k += 32) {
+                const double2 w = __ldcg(reinterpret_cast<const double2*>(part_b) + k);
+                sx += w.x;
+                sy += w.y;
+            }
+            sx = lane_sum(sx);
+            sy = lane_sum(sy);
             if (lane == 0) {
-                tot[1 + warp] = s;
-                if (!ok) arrived = 0;
+                tot[1] = sx;
+                tot[2] = sy;
             }
         }
         __syncthreads();
-        x = tot[1];
-        y = tot[2];
-        return arrived != 0;
+        tx = tot[1];
+        ty = tot[2];
+        return true;
     };
-    if (t == 0) arrived = 1;
     __syncthreads();
     double rz, rr, bnorm, tol, rr_stop = -1.0;
     long long it = 0, max_iter;
     int status = PCG_RUNNING;
-    bool ok = true;
     if constexpr (GRID) {
         volatile PcgScalars* s = a.s;
         rz = s->rz;
@@ -626,8 +560,7 @@ __global__ void __launch_bounds__(CH, 1) brick_pcg_kernel(BrickArgs a) {
     } else {
         tol = a.tol[inst];
         max_iter = a.max_iter[inst];
-        post_b(lrr, lrz, 1);
-        ok = total_b(rr, rz, 1);
+        sums_b(lrr, lrz, rr, rz);
         bnorm = sqrt(rr);
         if (bnorm == 0.0) status = PCG_CONVERGED;
     }
@@ -635,9 +568,7 @@ __global__ void __launch_bounds__(CH, 1) brick_pcg_kernel(BrickArgs a) {
     double surely = (tol * bnorm) * (tol * bnorm) * (1.0 + 1e-12);
     if (surely < 1e-280) surely = INFINITY;  // the square left the normal range
     __syncthreads();
-    unsigned long long seq = 1;
-    for (int step = 0; status == PCG_RUNNING && ok && (!GRID || step < a.chunk); ++step) {
-        seq += 1;
+    for (int step = 0; status == PCG_RUNNING && (!GRID || step < a.chunk); ++step) {
         const int64_t turn_at = (step & 1) * int64_t(b.bricks) * b.ncap;
         double* rows = a.rows + 4 * turn_at;
         auto share = [&](int l, const double (&q)[3]) {
@@ -719,26 +650,22 @@ __global__ void __launch_bounds__(CH, 1) brick_pcg_kernel(BrickArgs a) {
                     const double q[3] = {qs[3 * l], qs[3 * l + 1], qs[3 * l + 2]};
                     share(l, q);
                 }
-        // ---- exchange A: p.Kp; the partial forces are released with it
+        // ---- the CTAs meet: p.Kp, and the partial forces
         dot = lane_sum(dot);
         if (lane == 0) wa[warp] = dot;
         __syncthreads();
         if (warp == 0) {
             const double w = lane_sum(lane < WARPS ? wa[lane] : 0.0);
-            if (lane == 0) post_release(slot_a + (brick - brick0), w, seq);
+            if (lane == 0) part_a[brick - brick0] = w;
         }
-        if constexpr (!GRID) cluster_meet();
+        if (!meet()) return;
         if (warp == 0) {
-            double s;
-            const bool good = collect<GRID, GRID>(slot_a, 1, nb, seq, lane, s);
-            if (lane == 0) {
-                tot[0] = s;
-                if (!good) arrived = 0;
-            }
+            double s = 0.0;
+            for (int k = lane; k < nb; k += 32) s += __ldcg(part_a + k);
+            s = lane_sum(s);
+            if (lane == 0) tot[0] = s;
         }
         __syncthreads();
-        ok = arrived != 0;
-        if (!ok) break;
         const double pap = tot[0];
         if (!(pap > 0.0)) {  // p.Kp <= 0 or NaN: breakdown
             status = PCG_BREAKDOWN;
@@ -808,10 +735,9 @@ __global__ void __launch_bounds__(CH, 1) brick_pcg_kernel(BrickArgs a) {
                 }
             }
         }
-        // ---- exchange B: r.r and r.z
+        // ---- the CTAs meet: r.r and r.z
         double rz_new;
-        post_b(lrr, lrz, seq);
-        ok = total_b(rr, rz_new, seq);
+        if (!sums_b(lrr, lrz, rr, rz_new)) return;
         it += 1;
         if (!(rr > surely) && sqrt(rr) / bnorm <= tol) {
             status = PCG_CONVERGED;
@@ -841,7 +767,6 @@ __global__ void __launch_bounds__(CH, 1) brick_pcg_kernel(BrickArgs a) {
             }
         }
     }
-    if (t == 0 && !ok && GRID) atomicExch(&a.gb->error, 1);
     if (t == 0 && brick == brick0) {
         const double res = bnorm == 0.0 ? 0.0 : sqrt(rr) / bnorm;
         if constexpr (GRID) {
@@ -854,7 +779,7 @@ __global__ void __launch_bounds__(CH, 1) brick_pcg_kernel(BrickArgs a) {
         } else {
             a.out_it[inst] = it;
             a.out_res[inst] = res;
-            a.out_status[inst] = ok ? status : RESIDENT_STALLED;
+            a.out_status[inst] = status;
         }
     }
 }
@@ -996,7 +921,7 @@ BrickArgs brick_args(const svx_op* op, BrickWork& w) {
     a.fixed = op->is_fixed.p;
     a.inv_diag = op->inv_diag.p;
     a.rows = w.exchange.p;
-    a.slots = reinterpret_cast<Slot*>(w.slots.p);
+    a.part = w.part.p;
     a.rb = w.vec.p;
     if (w.vec.p) {
         const size_t n = size_t(op->brick.bricks) * op->brick.ncap * 3;
@@ -1010,7 +935,7 @@ BrickArgs brick_args(const svx_op* op, BrickWork& w) {
 void BrickWork::alloc(svx_ctx* ctx, const svx_op* op, bool single) {
     const BrickOperator& B = op->brick;
     exchange.alloc(ctx->pool, size_t(B.bricks) * B.ncap * 8);
-    slots.alloc(ctx->pool, size_t(B.bricks) * 6);
+    part.alloc(ctx->pool, size_t(B.bricks) * 3 + 4);
     if (!single) vec.alloc(ctx->pool, size_t(B.bricks) * B.ncap * 9);
     gb.alloc(ctx->pool, 1);
 }
@@ -1033,7 +958,6 @@ void brick_grid_launch(svx_ctx* ctx, const svx_op* op, BrickWork& w, double* u, 
     SVX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   int(BRICK_SMEM)));
     SVX_CUDA(cudaMemsetAsync(w.gb.p, 0, sizeof(GridBarrier), st));
-    SVX_CUDA(cudaMemsetAsync(w.slots.p, 0, w.slots.bytes(), st));
     void* args[] = {&a};
     SVX_CUDA(cudaLaunchCooperativeKernel(fn, dim3(unsigned(op->brick.bricks)),
                                          dim3(CH), args,

@@ -348,6 +348,7 @@ struct svx_op {
     // slot fastest: the shared-memory PCG kernel's operand (ndof >= 2)
     svx::DBuf<double> valsT;
     svx::DBuf<float> vals32;       // FP32 copy (mixed precision)
+    svx::DBuf<float> vals32T;      // that copy in valsT's layout (FP32 inner solves)
     // the FP32 copy in quads (3D operators, graph-form SpMV): node i's 9
     // (da, db) rows over its neighbour slots, slot fastest, padded to a
     // multiple of 4 slots, from baseq[i]; adjq its neighbours padded with
@@ -491,7 +492,7 @@ constexpr int BRICK_LAYERS = 1024;
 constexpr int BRICK_MAX_ELEMS = 2016;        // seven chunks; 16,384 references
 constexpr size_t BRICK_SMEM = 226 * 1024;    // of 227 KB, less the kernel's static arrays
 struct BrickWork {
-    DBuf<double> exchange, slots, vec;
+    DBuf<double> exchange, part, vec;
     DBuf<GridBarrier> gb;
     void alloc(svx_ctx* ctx, const svx_op* op, bool single);
 };

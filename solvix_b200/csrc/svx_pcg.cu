@@ -33,6 +33,7 @@
 
 #include "svx_internal.h"
 #include "svx_grid.h"
+#include "svx_warp.h"
 
 #include <cooperative_groups.h>
 
@@ -619,11 +620,10 @@ __global__ void compensated_fp32_kernel(int64_t n_nodes, const int64_t* __restri
 // da ND d + k ND + db) -> valsT, the same values of each node with the slot
 // fastest: (da ND + db) d + k.  One thread per (node, da, db); a node no
 // element uses keeps its ND diagonal values in place.
-template <int ND>
+template <int ND, class M>
 __global__ void transpose_blocks_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
                                         const int64_t* __restrict__ node_base,
-                                        const double* __restrict__ vals,
-                                        double* __restrict__ out) {
+                                        const M* __restrict__ vals, M* __restrict__ out) {
     const int64_t t = int64_t(blockIdx.x) * BLOCK + threadIdx.x;
     const int64_t i = t / (ND * ND);
     if (i >= n_nodes) return;
@@ -634,8 +634,8 @@ __global__ void transpose_blocks_kernel(int64_t n_nodes, const int64_t* __restri
         if (db == 0) out[base + da] = vals[base + da];
         return;
     }
-    const double* src = vals + base + int64_t(da) * ND * d + db;
-    double* dst = out + base + int64_t(da * ND + db) * d;
+    const M* src = vals + base + int64_t(da) * ND * d + db;
+    M* dst = out + base + int64_t(da * ND + db) * d;
     for (int k = 0; k < d; ++k) dst[k] = src[int64_t(k) * ND];
 }
 
@@ -1286,32 +1286,6 @@ pcg_persistent2_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
 // block sums the block partials in index order), so repeated runs are
 // bitwise identical.
 
-// Sums a, b over the block; every thread gets the totals.
-__device__ __forceinline__ void block_sum2(double& a, double& b, double* sh) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    a = warp_sum(a);
-    b = warp_sum(b);
-    __syncthreads();
-    if (lane == 0) {
-        sh[w] = a;
-        sh[32 + w] = b;
-    }
-    __syncthreads();
-    if (w == 0) {
-        double ta = lane < nw ? sh[lane] : 0.0;
-        double tb = lane < nw ? sh[32 + lane] : 0.0;
-        ta = warp_sum(ta);
-        tb = warp_sum(tb);
-        if (lane == 0) {
-            sh[0] = ta;
-            sh[32] = tb;
-        }
-    }
-    __syncthreads();
-    a = sh[0];
-    b = sh[32];
-}
-
 // The three-barrier form stages the p values its SpMV gathers: the window of
 // nodes [lowest, highest neighbour of the block's nodes] is copied from L2
 // into shared memory once an iteration (coalesced), instead of every node
@@ -1323,80 +1297,93 @@ __device__ __forceinline__ void block_sum2(double& a, double& b, double* sh) {
 // 25.4 us an iteration gathering from L2, both with 32 lanes a node.)
 constexpr int STAGE_NODES_PER_NODE = 4;
 
-__host__ __device__ inline size_t smem_adj_offset(int64_t nodes_cap, int nd) {
-    return size_t(nodes_cap) * size_t(nd) * 8 * 6;
+__host__ __device__ inline size_t smem_adj_offset(int64_t nodes_cap, int nd, size_t value) {
+    return size_t(nodes_cap) * size_t(nd) * value * 6;
 }
 
 // Dynamic shared memory of pcg_smem_kernel for `nodes_cap` nodes of `nd`
 // dofs and at most max_deg neighbours: six vectors of nodes_cap * nd
-// doubles, the adjacency in load_shared_adj's layout (rounded up to 16
+// values of `value` bytes, the adjacency in load_shared_adj's layout (rounded up to 16
 // bytes), then the staging window of stage_nodes nodes.
-size_t smem_pcg_bytes(int64_t nodes_cap, int nd, int max_deg, int64_t stage_nodes) {
+size_t smem_pcg_bytes(int64_t nodes_cap, int nd, int max_deg, int64_t stage_nodes, size_t value) {
     const size_t adj = (shared_adj_bytes(nodes_cap, max_deg) + 15) / 16 * 16;
-    return smem_adj_offset(nodes_cap, nd) + adj + size_t(stage_nodes) * size_t(nd) * 8;
+    return smem_adj_offset(nodes_cap, nd, value) + adj + size_t(stage_nodes) * size_t(nd) * value;
 }
 
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
 // The gathered value of column c: p_c itself (ALG 0) or z_c + beta pprev_c
-// formed with one fused multiply-add (ALG 1).
+// formed with one fused multiply-add of the vectors' type (ALG 1).
 // XS: x is the shared-memory staging window of the nodes from xoff / ND on.
-template <int ALG, bool XS>
-__device__ __forceinline__ double gathered(const double* x, const double* z, const double* pprev,
-                                           double beta, int64_t c, int64_t xoff) {
+template <int ALG, bool XS, class V>
+__device__ __forceinline__ double gathered(const V* x, const V* z, const V* pprev, V beta,
+                                           int64_t c, int64_t xoff) {
     if constexpr (ALG == 0) {
-        if constexpr (XS) return x[c - xoff];
-        else return __ldcg(x + c);
+        if constexpr (XS) return double(x[c - xoff]);
+        else return double(__ldcg(x + c));
     }
-    return __fma_rn(beta, __ldcg(pprev + c), __ldcg(z + c));
+    return double(fma_rn(beta, __ldcg(pprev + c), __ldcg(z + c)));
 }
 
 // One node's rows, lane gl of its G-lane group taking neighbour blocks gl,
-// gl + G, ...  The values come from the transposed copy valsT (entry
-// (da, db) of neighbour slot k at (da ND + db) d + k from the node's base),
-// so the loads of one (da, db) by the lanes of a group are consecutive
-// doubles, where in the row layout they stride ND doubles.  The first
-// block is loaded under a predicate rather than a branch, so that the U
-// nodes of a warp step issue its loads before their first multiply-add;
-// the blocks past the first G (a C3D8 node's 27 at G = 8) loop.
-template <int ND, int G, int ALG, bool XS>
-__device__ __forceinline__ void node_rows_pred(bool valid, const int32_t* cols, int d,
-                                               const double* v, const double* x,
-                                               const double* z, const double* pprev,
-                                               double beta, int64_t i, int gl, double* acc,
-                                               int64_t xoff) {
+// gl + G, ...  The values come from the transposed copy (entry (da, db) of
+// neighbour slot k at (da ND + db) d + k from the node's base), so the loads
+// of one (da, db) by the lanes of a group are consecutive values, where in
+// the row layout they stride ND.  The first block is loaded under a
+// predicate rather than a branch, so that the U nodes of a warp step issue
+// its loads before their first multiply-add; the blocks past the first G (a
+// C3D8 node's 27 at G = 8) loop.  An FP32 operator is in difference form:
+// the node's own x (own) is taken from every other neighbour's.
+template <int ND, int G, int ALG, bool XS, class M, class V>
+__device__ __forceinline__ void node_rows_pred(bool valid, const int32_t* cols, int d, const M* v,
+                                               const V* x, const V* z, const V* pprev, V beta,
+                                               int64_t i, int gl, double* acc, int64_t xoff,
+                                               const V* own) {
+    constexpr bool DIFF = std::is_same<M, float>::value;
     const bool act = valid && gl < d;
-    const int64_t c0 = int64_t(act ? cols[gl] : 0) * ND;
-    double xv[ND];
+    const int32_t j0 = act ? cols[gl] : 0;
+    const int64_t c0 = int64_t(j0) * ND;
+    double xv[ND], xi[ND];
 #pragma unroll
-    for (int db = 0; db < ND; ++db) xv[db] = act ? gathered<ALG, XS>(x, z, pprev, beta, c0 + db, xoff) : 0.0;
+    for (int db = 0; db < ND; ++db) {
+        xv[db] = act ? gathered<ALG, XS>(x, z, pprev, beta, c0 + db, xoff) : 0.0;
+        xi[db] = DIFF ? double(own[db]) : 0.0;
+        if (DIFF && act && j0 != int32_t(i)) xv[db] -= xi[db];
+    }
 #pragma unroll
     for (int da = 0; da < ND; ++da)
 #pragma unroll
         for (int db = 0; db < ND; ++db)
-            acc[da] += (act ? __ldg(v + (da * ND + db) * d + gl) : 0.0) * xv[db];
+            acc[da] += (act ? double(__ldg(v + (da * ND + db) * d + gl)) : 0.0) * xv[db];
     if (valid && d > G) {
         for (int k = gl + G; k < d; k += G) {
-            const int64_t c = int64_t(cols[k]) * ND;
+            const int32_t j = cols[k];
+            const int64_t c = int64_t(j) * ND;
 #pragma unroll
-            for (int db = 0; db < ND; ++db) xv[db] = gathered<ALG, XS>(x, z, pprev, beta, c + db, xoff);
+            for (int db = 0; db < ND; ++db) {
+                xv[db] = gathered<ALG, XS>(x, z, pprev, beta, c + db, xoff);
+                if (DIFF && j != int32_t(i)) xv[db] -= xi[db];
+            }
 #pragma unroll
             for (int da = 0; da < ND; ++da)
 #pragma unroll
                 for (int db = 0; db < ND; ++db)
-                    acc[da] += __ldg(v + (da * ND + db) * d + k) * xv[db];
+                    acc[da] += double(__ldg(v + (da * ND + db) * d + k)) * xv[db];
         }
     }
     if (valid && d == 0 && gl == 0)  // an unreferenced node: rows of length 1
 #pragma unroll
         for (int da = 0; da < ND; ++da)
-            acc[da] = v[da] * gathered<ALG, XS>(x, z, pprev, beta, i * ND + da, xoff);
+            acc[da] = double(v[da]) * gathered<ALG, XS>(x, z, pprev, beta, i * ND + da, xoff);
 }
 
-template <int ND, int G, int PB, int BPS, int ALG, int U>
+template <int ND, int G, int PB, int BPS, int ALG, int U, class M, class V>
 __global__ void __launch_bounds__(PB, BPS)
 pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
                 const int32_t* __restrict__ adj, const int64_t* __restrict__ node_base,
-                const double* __restrict__ vals, const double* __restrict__ inv_diag,
-                double* u_g, double* r_g, double* p_g, double* p2_g, double* z_g,
+                const M* __restrict__ vals, const V* __restrict__ inv_diag,
+                V* u_g, V* r_g, V* p_g, V* p2_g, V* z_g,
                 double* part, PcgScalars* s, GridBarrier* gb, int chunk, int nodes_cap,
                 int max_deg, int stage, int first) {
     extern __shared__ __align__(16) unsigned char svx_dyn_smem[];
@@ -1416,19 +1403,19 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
     const int nb1 = int(n_nodes * int64_t(blockIdx.x + 1) / B);
     const int nloc = nb1 - nb0, rows = nloc * ND, row0 = nb0 * ND;
     const int rcap = nodes_cap * ND;
-    double* u_s = reinterpret_cast<double*>(svx_dyn_smem);
-    double* r_s = u_s + rcap;
-    double* p_s = r_s + rcap;
-    double* q_s = p_s + rcap;
-    double* z_s = q_s + rcap;
-    double* d_s = z_s + rcap;
+    V* u_s = reinterpret_cast<V*>(svx_dyn_smem);
+    V* r_s = u_s + rcap;
+    V* p_s = r_s + rcap;
+    V* q_s = p_s + rcap;
+    V* z_s = q_s + rcap;
+    V* d_s = z_s + rcap;
     const SharedAdj sa = load_shared_adj_at(reinterpret_cast<unsigned char*>(d_s + rcap),
                                             adj_ptr, adj, node_base, nb0, nb1, nodes_cap);
     // the staging window (three-barrier form): nodes [jlo, jhi] of every
     // column the block's rows reach, its own nodes included
     __shared__ int s_jlo, s_jhi;
-    double* xs = reinterpret_cast<double*>(
-        svx_dyn_smem + smem_adj_offset(nodes_cap, ND) +
+    V* xs = reinterpret_cast<V*>(
+        svx_dyn_smem + smem_adj_offset(nodes_cap, ND, sizeof(V)) +
         (shared_adj_bytes(nodes_cap, max_deg) + 15) / 16 * 16);
     bool staged = false;
     int jlo = 0, jhi = -1;
@@ -1462,18 +1449,18 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
     double rz = vs->rz, beta = vs->beta;
     // ALG 1 alternates the previous-p buffers: iteration it reads p_{it-1}
     // from buf(it) and writes p_it to buf(it + 1)
-    auto buf = [&](long long k) -> double* { return (k & 1) ? p2_g : p_g; };
+    auto buf = [&](long long k) -> V* { return (k & 1) ? p2_g : p_g; };
     for (int t = threadIdx.x; t < rows; t += PB) {
         const int row = row0 + t;
-        const double di = inv_diag[row];
-        const double ri = r_g[row];
+        const V di = inv_diag[row];
+        const V ri = r_g[row];
         d_s[t] = di;
         r_s[t] = ri;
         z_s[t] = ri * di;
         u_s[t] = u_g[row];
         // the first launch starts from p = z (the init kernel's p); later
         // launches from the stored direction
-        p_s[t] = ALG == 1 ? (first ? 0.0 : buf(it)[row]) : p_g[row];
+        p_s[t] = ALG == 1 ? (first ? V(0) : buf(it)[row]) : p_g[row];
     }
     if (ALG == 1 && first) beta = 0.0;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1481,38 +1468,54 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
     const int gl = lane & (G - 1), grp = lane / G;
     const bool writer = (blockIdx.x == 0 && threadIdx.x == 0);
     __syncthreads();
-    if (ALG == 1 && first) {
-        // neighbours gather z and the previous p (zero): store z, barrier
-        for (int t = threadIdx.x; t < rows; t += PB) {
-            z_g[row0 + t] = z_s[t];
-            p_g[row0 + t] = 0.0;
-        }
-        if (!grid_sync(gb, B, bar_target)) return;
-    }
-
     // sum over the grid of the block partials (a, b), published in slot
     // `slot` of `part`.  The two reductions of an iteration use two slots: a
     // block past the first one's barrier may publish its second partials
     // while a late block still reads the first ones; with a barrier between
     // two uses of a slot no block can overwrite what another still reads.
+    // Warp sums on the tensor cores, and one warp reads the other blocks'
+    // partials: read by all 16 warps of 148 blocks their few cache lines are
+    // a hot spot of the L2.  (Posting the sums as numbered words that every
+    // block polls, instead of the counting barrier, measured slower: 8.8
+    // against 7.2 us an iteration at 81 nodes, 12.4 against 8.2 at 6,561.)
     auto grid_totals = [&](int slot, double a, double b, double& ta, double& tb) -> bool {
         double* pt = part + size_t(slot) * 2 * B;
-        block_sum2(a, b, sh);
-        if (threadIdx.x == 0) {
-            pt[2 * blockIdx.x] = a;
-            pt[2 * blockIdx.x + 1] = b;
+        const double v = lane_sum_pair(a, b, lane);
+        if ((lane & 15) == 0) sh[2 * warp + (lane >> 4)] = v;
+        __syncthreads();
+        if (warp == 0) {
+            const double w = lane_sum_pair(lane < W ? sh[2 * lane] : 0.0,
+                                           lane < W ? sh[2 * lane + 1] : 0.0, lane);
+            if ((lane & 15) == 0) pt[2 * blockIdx.x + (lane >> 4)] = w;
         }
         if (!grid_sync(gb, B, bar_target)) return false;
-        double x = 0.0, y = 0.0;
-        for (int k = threadIdx.x; k < int(B); k += PB) {
-            x += __ldcg(pt + 2 * k);
-            y += __ldcg(pt + 2 * k + 1);
+        if (warp == 0) {
+            double x = 0.0, y = 0.0;
+            for (int k = lane; k < int(B); k += 32) {
+                const double2 w = __ldcg(reinterpret_cast<const double2*>(pt) + k);
+                x += w.x;
+                y += w.y;
+            }
+            x = lane_sum(x);
+            y = lane_sum(y);
+            if (lane == 0) {
+                sh[32] = x;
+                sh[33] = y;
+            }
         }
-        block_sum2(x, y, sh);
-        ta = x;
-        tb = y;
+        __syncthreads();
+        ta = sh[32];
+        tb = sh[33];
         return true;
     };
+    if (ALG == 1 && first) {
+        // neighbours gather z and the previous p (zero): store z, barrier
+        for (int t = threadIdx.x; t < rows; t += PB) {
+            z_g[row0 + t] = z_s[t];
+            p_g[row0 + t] = V(0);
+        }
+        if (!grid_sync(gb, B, bar_target)) return;
+    }
     auto finish = [&](int status) {
         for (int t = threadIdx.x; t < rows; t += PB) {
             const int row = row0 + t;
@@ -1533,8 +1536,9 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
 
     for (int c = 0; c < chunk; ++c) {
         // q = K p on the block's nodes, p.q on its rows
-        const double* pprev = buf(it);
-        double* pnext = buf(it + 1);
+        const V* pprev = buf(it);
+        V* pnext = buf(it + 1);
+        const V bt = V(beta);
         if (ALG == 0) {
             for (int t = threadIdx.x; t < rows; t += PB) p_g[row0 + t] = p_s[t];
             if (!grid_sync(gb, B, bar_target)) return;
@@ -1545,10 +1549,11 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
             }
         } else {
             for (int t = threadIdx.x; t < rows; t += PB) {
-                const double pi = __fma_rn(beta, p_s[t], z_s[t]);
+                const V pi = fma_rn(bt, p_s[t], z_s[t]);
                 p_s[t] = pi;
                 pnext[row0 + t] = pi;
             }
+            if (std::is_same<M, float>::value) __syncthreads();  // rows read their own p
         }
         // U steps of the warp's nodes at a time, all their loads in flight
         const int steps = (wn1 - wn0 + NPS - 1) / NPS;
@@ -1565,12 +1570,14 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
                 for (int da = 0; da < ND; ++da) acc[uu][da] = 0.0;
                 const int64_t vb = valid ? sa.vbase[li] : 0;
                 if (staged)
-                    node_rows_pred<ND, G, ALG, true>(valid, sa.cols + a0, d, vals + vb, xs, z_g,
-                                                     pprev, beta, i, gl, acc[uu],
-                                                     int64_t(jlo) * ND);
+                    node_rows_pred<ND, G, ALG, true>(valid, sa.cols + a0, d, vals + vb,
+                                                     (const V*)xs, (const V*)z_g, pprev, bt, i, gl,
+                                                     acc[uu], int64_t(jlo) * ND,
+                                                     (const V*)p_s + li * ND);
                 else
-                    node_rows_pred<ND, G, ALG, false>(valid, sa.cols + a0, d, vals + vb, p_g,
-                                                      z_g, pprev, beta, i, gl, acc[uu], 0);
+                    node_rows_pred<ND, G, ALG, false>(valid, sa.cols + a0, d, vals + vb,
+                                                      (const V*)p_g, (const V*)z_g, pprev, bt, i,
+                                                      gl, acc[uu], 0, (const V*)p_s + li * ND);
             }
 #pragma unroll
             for (int uu = 0; uu < U; ++uu)
@@ -1584,13 +1591,13 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
 #pragma unroll
                     for (int da = 1; da < ND; ++da)
                         if (gl == da) qi = acc[uu][da];
-                    q_s[(i - nb0) * ND + gl] = qi;
+                    q_s[(i - nb0) * ND + gl] = V(qi);
                 }
             }
         }
         __syncthreads();
         double pq = 0.0, zero = 0.0;
-        for (int t = threadIdx.x; t < rows; t += PB) pq += p_s[t] * q_s[t];
+        for (int t = threadIdx.x; t < rows; t += PB) pq += double(p_s[t]) * double(q_s[t]);
         double pap, unused;
         if (!grid_totals(0, pq, zero, pap, unused)) return;
         if (!(pap > 0.0)) {  // p.Kp <= 0 or NaN: breakdown
@@ -1599,18 +1606,18 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
             finish(PCG_BREAKDOWN);
             return;
         }
-        const double alpha = rz / pap;
+        const V alpha = V(rz / pap);
         // u += alpha p, r -= alpha q, z = r / K_ii; r.r, r.z
         double lrr = 0.0, lrz = 0.0;
         for (int t = threadIdx.x; t < rows; t += PB) {
             u_s[t] += alpha * p_s[t];
-            const double ri = r_s[t] - alpha * q_s[t];
-            const double zi = ri * d_s[t];
+            const V ri = r_s[t] - alpha * q_s[t];
+            const V zi = ri * d_s[t];
             r_s[t] = ri;
             z_s[t] = zi;
             if (ALG == 1) z_g[row0 + t] = zi;
-            lrr += ri * ri;
-            lrz += ri * zi;
+            lrr += double(ri) * double(ri);
+            lrz += double(ri) * double(zi);
         }
         double rr, rz_new;
         if (!grid_totals(1, lrr, lrz, rr, rz_new)) return;
@@ -1629,7 +1636,7 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
         beta = rz_new / rz;
         rz = rz_new;
         if (ALG == 0)
-            for (int t = threadIdx.x; t < rows; t += PB) p_s[t] = z_s[t] + beta * p_s[t];
+            for (int t = threadIdx.x; t < rows; t += PB) p_s[t] = z_s[t] + V(beta) * p_s[t];
     }
     finish(PCG_RUNNING);
 }
@@ -2496,9 +2503,8 @@ struct PcgRun {
     // block's rows and adjacency do not fit its shared memory (the caller
     // then runs the register-vector persistent kernel).
     // valsT: K in the transposed node-block layout (transposed_values)
-    int iterate_smem(int chunk, const double* valsT) {
-        if constexpr (!(std::is_same<M, double>::value && std::is_same<V, double>::value &&
-                        std::is_same<U, double>::value)) {
+    int iterate_smem(int chunk, const M* valsT) {
+        if constexpr (!(std::is_same<M, V>::value && std::is_same<V, U>::value)) {
             (void)chunk;
             (void)valsT;
             return -1;
@@ -2542,20 +2548,29 @@ struct PcgRun {
 #define SVX_SMEM_PICK(ND_, G_)                                                           \
     if (ND == ND_ && G == G_) {                                                          \
         if (alg == 0) {                                                                  \
-            if (unroll == 1) return (void*)pcg_smem_kernel<ND_, G_, PB, 1, 0, 1>;        \
-            if (unroll == 2) return (void*)pcg_smem_kernel<ND_, G_, PB, 1, 0, 2>;        \
-            return (void*)pcg_smem_kernel<ND_, G_, PB, 1, 0, 4>;                         \
+            if (unroll == 1) return (void*)pcg_smem_kernel<ND_, G_, PB, 1, 0, 1, M, V>;        \
+            if (unroll == 2) return (void*)pcg_smem_kernel<ND_, G_, PB, 1, 0, 2, M, V>;        \
+            return (void*)pcg_smem_kernel<ND_, G_, PB, 1, 0, 4, M, V>;                         \
         }                                                                                \
-        if (unroll == 1) return (void*)pcg_smem_kernel<ND_, G_, PB, 1, 1, 1>;            \
-        if (unroll == 2) return (void*)pcg_smem_kernel<ND_, G_, PB, 1, 1, 2>;            \
-        return (void*)pcg_smem_kernel<ND_, G_, PB, 1, 1, 4>;                             \
+        if (unroll == 1) return (void*)pcg_smem_kernel<ND_, G_, PB, 1, 1, 1, M, V>;            \
+        if (unroll == 2) return (void*)pcg_smem_kernel<ND_, G_, PB, 1, 1, 2, M, V>;            \
+        return (void*)pcg_smem_kernel<ND_, G_, PB, 1, 1, 4, M, V>;                             \
     }
-                SVX_SMEM_PICK(3, 32)
-                SVX_SMEM_PICK(3, 8)
-                SVX_SMEM_PICK(2, 16)
-                SVX_SMEM_PICK(2, 8)
-                SVX_SMEM_PICK(1, 16)
-                SVX_SMEM_PICK(1, 8)
+                if constexpr (std::is_same<M, float>::value) {
+                    // FP32 inner solves: the default shapes
+                    if (ND == 3)
+                        return alg == 0 ? (void*)pcg_smem_kernel<3, 8, PB, 1, 0, 1, M, V>
+                                        : (void*)pcg_smem_kernel<3, 8, PB, 1, 1, 1, M, V>;
+                    if (ND == 2) return (void*)pcg_smem_kernel<2, 8, PB, 1, 1, 1, M, V>;
+                    return nullptr;
+                } else {
+                    SVX_SMEM_PICK(3, 32)
+                    SVX_SMEM_PICK(3, 8)
+                    SVX_SMEM_PICK(2, 16)
+                    SVX_SMEM_PICK(2, 8)
+                    SVX_SMEM_PICK(1, 16)
+                    SVX_SMEM_PICK(1, 8)
+                }
 #undef SVX_SMEM_PICK
                 return nullptr;
             };
@@ -2567,11 +2582,11 @@ struct PcgRun {
             cudaFuncAttributes fa{};
             SVX_CUDA(cudaFuncGetAttributes(&fa, fn));
             const size_t avail = size_t(max_smem) - std::min(size_t(max_smem), fa.sharedSizeBytes);
-            const size_t base = smem_pcg_bytes(nodes_cap, ND, op->pat.max_deg, 0);
+            const size_t base = smem_pcg_bytes(nodes_cap, ND, op->pat.max_deg, 0, sizeof(V));
             if (base > avail) return -1;
             // the three-barrier form's staging window
             int stage = (alg == 0 && ctx->pcg_stage) ? STAGE_NODES_PER_NODE * nodes_cap : 0;
-            const size_t smem = smem_pcg_bytes(nodes_cap, ND, op->pat.max_deg, stage);
+            const size_t smem = smem_pcg_bytes(nodes_cap, ND, op->pat.max_deg, stage, sizeof(V));
             if (smem > avail) return -1;
             SVX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           int(smem)));
@@ -2580,7 +2595,8 @@ struct PcgRun {
             if (bps < 1) return -1;
             const int pb = PB;
             if (!fn) return -1;
-            DBuf<double> part, z;
+            DBuf<double> part;
+            DBuf<V> z;
             DBuf<GridBarrier> gb;
             part.alloc(ctx->pool, 4 * size_t(B) + 2);  // two slots of pairs
             z.alloc(ctx->pool, n + 1);
@@ -2592,7 +2608,7 @@ struct PcgRun {
             const int64_t* nbase = op->pat.node_base.p;
             GridBarrier* gbp = gb.p;
             double* pp = part.p;
-            double* zp = z.p;
+            V* zp = z.p;
             int first = 1;
             int max_deg = std::max(op->pat.max_deg, 1);
             if (!p2) return -1;
@@ -2758,22 +2774,26 @@ int auto_check_every(int64_t n, int64_t nnz) {
 
 // The transposed copy of K the shared-memory PCG kernel streams (vectors of
 // one dof per node need none: both layouts are the same).
-const double* transposed_values(svx_ctx* ctx, svx_op* op) {
-    if (op->ndof == 1) return op->vals.p;
-    if (!op->valsT.p) {
-        op->valsT.alloc(ctx->pool, op->pat.nnz + 1);
+template <class M>
+static const M* transposed(svx_ctx* ctx, const svx_op* op, const DBuf<M>& vals, DBuf<M>& out) {
+    if (op->ndof == 1) return vals.p;
+    if (!out.p) {
+        out.alloc(ctx->pool, op->pat.nnz + 1);
         const int64_t threads = op->n_nodes * op->ndof * op->ndof;
         const unsigned grid = unsigned(std::max<int64_t>(1, (threads + BLOCK - 1) / BLOCK));
         const Pattern& P = op->pat;
         if (op->ndof == 3)
-            transpose_blocks_kernel<3><<<grid, BLOCK, 0, ctx->stream>>>(
-                op->n_nodes, P.adj_ptr.p, P.node_base.p, op->vals.p, op->valsT.p);
+            transpose_blocks_kernel<3, M><<<grid, BLOCK, 0, ctx->stream>>>(
+                op->n_nodes, P.adj_ptr.p, P.node_base.p, vals.p, out.p);
         else
-            transpose_blocks_kernel<2><<<grid, BLOCK, 0, ctx->stream>>>(
-                op->n_nodes, P.adj_ptr.p, P.node_base.p, op->vals.p, op->valsT.p);
+            transpose_blocks_kernel<2, M><<<grid, BLOCK, 0, ctx->stream>>>(
+                op->n_nodes, P.adj_ptr.p, P.node_base.p, vals.p, out.p);
         SVX_LAUNCH_CHECK();
     }
-    return op->valsT.p;
+    return out.p;
+}
+const double* transposed_values(svx_ctx* ctx, svx_op* op) {
+    return transposed(ctx, op, op->vals, op->valsT);
 }
 
 void build_fp32_operator(svx_ctx* ctx, svx_op* op) {
@@ -2944,8 +2964,8 @@ static PcgResult pcg_resident(svx_ctx* ctx, svx_op* op, const ResidentShape& sha
 
 // Gives an FP64 run of a C3D8 model its element-by-element form, where it
 // has one: bricks while a model's bricks fit the chip, the graph form above.
-static void wire_hex(svx_ctx* ctx, svx_op* op, PcgRun<double, double, double>& run, HexWork& hex,
-                     BrickWork& brick) {
+static void wire_hex_form(svx_ctx* ctx, svx_op* op, PcgRun<double, double, double>& run,
+                          HexWork& hex, BrickWork& brick) {
     if (!hex_applies(ctx, op)) return;
     if (!(ctx->graph_min_nnz >= 0 && use_graph_form(ctx, op)) && op->brick.state == 0) {
         int coop = 0;
@@ -2969,6 +2989,24 @@ static void wire_hex(svx_ctx* ctx, svx_op* op, PcgRun<double, double, double>& r
     hex_prepare(ctx, op);
     hex.alloc(ctx, op);
     run.hex = &hex;
+}
+
+// A device too full for the form's own arrays (about a sixth of the assembled
+// K) solves on K, as it could before.
+static void wire_hex(svx_ctx* ctx, svx_op* op, PcgRun<double, double, double>& run, HexWork& hex,
+                     BrickWork& brick) {
+    try {
+        wire_hex_form(ctx, op, run, hex, brick);
+    } catch (const ModelFail& f) {
+        if (f.code != SVX_OOM) throw;
+        SVX_CUDA(cudaStreamSynchronize(ctx->stream));
+        run.hex = nullptr;
+        run.brick = nullptr;
+        hex = HexWork{};
+        brick = BrickWork{};
+        op->hex = HexOperator{};
+        op->brick = BrickOperator{};
+    }
 }
 
 PcgResult pcg_fp64(svx_ctx* ctx, svx_op* op, double tol, long long max_iter, int check_every,
@@ -3334,7 +3372,7 @@ PcgResult pcg_defect_correction(svx_ctx* ctx, svx_op* op, double tol, long long 
     build_fp32_operator(ctx, op);
     const int G = pick_node_group(op->pat.max_deg, op->ndof);
     const unsigned grid_r = grid_nodes(ctx, op->n_nodes, G), grid_v = grid_vec(ctx, n);
-    DBuf<float> r32, p32, q32, e32, d32;
+    DBuf<float> r32, p32, q32, e32, d32, p2;
     DBuf<double> r64, e64, r, p, q, partials, rr_dev;
     DBuf<PcgScalars> s;
     DBuf<unsigned int> counter;
@@ -3392,6 +3430,20 @@ PcgResult pcg_defect_correction(svx_ctx* ctx, svx_op* op, double tol, long long 
         SVX_CUDA(cudaMemcpyAsync(hs.h, s.p, sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
         SVX_CUDA(cudaStreamSynchronize(st));
         int status = hs.h->status;
+        // below the graph threshold the shared-memory kernel runs the FP32
+        // inner solve too: in the graph its three launches' gaps cost more than
+        // the arithmetic (80 x 8 x 8: 14.8 us an iteration in the graph, 7.9
+        // here; 160 x 16 x 16: 23.3 and 17.4)
+        if constexpr (std::is_same<V, float>::value) {
+            if (status == PCG_RUNNING && !use_graph_form(ctx, op) && ctx->pcg_smem) {
+                if (!p2.p) p2.alloc(ctx->pool, n + 1);
+                SVX_CUDA(cudaMemsetAsync(p2.p, 0, (n + 1) * sizeof(float), st));
+                run.p2 = p2.p;
+                const int got = run.iterate_smem(persistent_chunk(op->pat.nnz),
+                                                 transposed(ctx, op, op->vals32, op->vals32T));
+                if (got >= 0) status = got;
+            }
+        }
         if (status == PCG_RUNNING) status = run.iterate(check_every);
         SVX_CUDA(cudaMemcpyAsync(hs.h, s.p, sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
         SVX_CUDA(cudaStreamSynchronize(st));
@@ -3845,6 +3897,7 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
     }
     // FP64 C3D8 members on bricks, a cluster of 1, 2, 4, 8 or 16 CTAs each
     std::vector<int> nbricks;
+    BrickWork brick;
     if (op->ndof == 3 && !mixed && ctx->hex && op->all_hex) {
         nbricks.assign(count, 0);
         bool any = false;
@@ -3858,7 +3911,18 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
             nbricks[k] = c;
             any = true;
         }
-        if (any) brick_build(ctx, op, false, node_off, elem_off, nbricks);
+        if (any) {
+            try {
+                brick_build(ctx, op, false, node_off, elem_off, nbricks);
+                brick.alloc(ctx, op, false);
+            } catch (const ModelFail& f) {  // a full device: the members solve on K
+                if (f.code != SVX_OOM) throw;
+                SVX_CUDA(cudaStreamSynchronize(st));
+                brick = BrickWork{};
+                op->brick = BrickOperator{};
+                std::fill(nbricks.begin(), nbricks.end(), 0);
+            }
+        }
         for (int k = 0; any && k < count; ++k)
             if (nbricks[k]) {
                 shapes.resize(count);
@@ -3985,11 +4049,6 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
         SVX_CUDA(cudaEventRecord(ctx->join_ev, ctx->aux_stream));
     }
     int n_class = 0;
-    BrickWork brick;
-    if (op->ndof == 3 && n_general < count) {
-        brick.alloc(ctx, op, false);
-        SVX_CUDA(cudaMemsetAsync(brick.slots.p, 0, brick.slots.bytes(), pst));
-    }
     for (int k0 = n_general; k0 < count; ++n_class) {
         // the run of members of one shape, its window the largest of them
         ResidentShape shape = shapes[ordered[k0]];

@@ -114,3 +114,17 @@ def test_batch_members_of_one_to_sixteen_ctas(ctx):
         alone, _ = ctx.solve_batch([flats[k]])
         assert np.array_equal(alone[0]["u"], out[k]["u"])
         assert alone[0]["iterations"] == out[k]["iterations"]
+
+
+@pytest.mark.parametrize("size", [(3, 1, 1), (20, 5, 4), (48, 9, 8)])
+def test_defect_correction_below_the_graph_threshold(ctx, size):
+    """The FP32 inner solves on the shared-memory kernel, of one node a block
+    to several (and the plane form's two barriers)."""
+    flat = block(*size, hetero=(9.0, 11.0))
+    sol, ref = ctx.solve_flat(flat, precision=abi.SVX_MIXED_DEFECT), oracle.solve_flat(flat)
+    assert sol.final_residual <= 1e-10 and 0 < sol.fp32_iterations <= sol.iterations
+    assert rel(sol.u, ref.u) <= 1e-8
+    plane = workloads.cantilever_cps4(10 * size[1], 4 * size[2], length=size[1],
+                                      height=0.4 * size[2])
+    sol = ctx.solve_flat(plane, precision=abi.SVX_MIXED_DEFECT)
+    assert rel(sol.u, oracle.solve_flat(plane).u) <= 1e-8
