@@ -1389,8 +1389,9 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
     extern __shared__ __align__(16) unsigned char svx_dyn_smem[];
     __shared__ double sh[64];
     // block-uniform values kept out of registers: ||f||, tol, the last
-    // iterate's ||r|| / ||f|| and r.r (thread 0 keeps them), max_iter
-    __shared__ double s_c[4];
+    // iterate's ||r|| / ||f|| and r.r (thread 0 keeps them), the reliable
+    // update's r.r, max_iter
+    __shared__ double s_c[5];
     __shared__ long long s_max_iter;
     constexpr int NPS = 32 / G;  // nodes per warp step
     constexpr int W = PB / 32;
@@ -1443,6 +1444,7 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
         s_c[1] = vs->tol;
         s_c[2] = vs->res;
         s_c[3] = vs->rr;
+        s_c[4] = vs->rr_stop;
         s_max_iter = vs->max_iter;
     }
     long long it = vs->it;
@@ -1631,6 +1633,10 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
             if (ALG == 1) beta = rz_new / rz;  // the next p of a resumed solve
             rz = rz_new;
             finish(res <= s_c[1] ? PCG_CONVERGED : PCG_MAXITER);
+            return;
+        }
+        if (rr <= s_c[4]) {  // rz stays r.z of the previous iterate
+            finish(PCG_RELIABLE);
             return;
         }
         beta = rz_new / rz;
@@ -2503,8 +2509,8 @@ struct PcgRun {
     // block's rows and adjacency do not fit its shared memory (the caller
     // then runs the register-vector persistent kernel).
     // valsT: K in the transposed node-block layout (transposed_values)
-    int iterate_smem(int chunk, const M* valsT) {
-        if constexpr (!(std::is_same<M, V>::value && std::is_same<V, U>::value)) {
+    int iterate_smem(int chunk, const M* valsT, int form = -1) {
+        if constexpr (!std::is_same<V, U>::value) {
             (void)chunk;
             (void)valsT;
             return -1;
@@ -2542,7 +2548,8 @@ struct PcgRun {
             const unsigned int B = unsigned(ctx->sm_count);
             const int nodes_cap = int((op->n_nodes + B - 1) / B);
             const int alg =
-                ctx->pcg_alg >= 0 ? ctx->pcg_alg : ((ND <= 2 || nodes_cap <= 64) ? 1 : 0);
+                form >= 0           ? form
+                : ctx->pcg_alg >= 0 ? ctx->pcg_alg : ((ND <= 2 || nodes_cap <= 64) ? 1 : 0);
             const int unroll = ctx->pcg_unroll > 0 ? ctx->pcg_unroll : 1;
             auto kernel_for = [&]() -> void* {
 #define SVX_SMEM_PICK(ND_, G_)                                                           \
@@ -2557,11 +2564,15 @@ struct PcgRun {
         return (void*)pcg_smem_kernel<ND_, G_, PB, 1, 1, 4, M, V>;                             \
     }
                 if constexpr (std::is_same<M, float>::value) {
-                    // FP32 inner solves: the default shapes
+                    // FP32 operators: the default shapes (FP64 vectors, the mixed
+                    // form, three barriers only)
+                    if (ND == 3 && std::is_same<V, double>::value)
+                        return (void*)pcg_smem_kernel<3, 8, PB, 1, 0, 1, M, V>;
                     if (ND == 3)
                         return alg == 0 ? (void*)pcg_smem_kernel<3, 8, PB, 1, 0, 1, M, V>
                                         : (void*)pcg_smem_kernel<3, 8, PB, 1, 1, 1, M, V>;
-                    if (ND == 2) return (void*)pcg_smem_kernel<2, 8, PB, 1, 1, 1, M, V>;
+                    if (ND == 2 && std::is_same<V, float>::value)
+                        return (void*)pcg_smem_kernel<2, 8, PB, 1, 1, 1, M, V>;
                     return nullptr;
                 } else {
                     SVX_SMEM_PICK(3, 32)
@@ -3238,10 +3249,22 @@ PcgResult pcg_mixed(svx_ctx* ctx, svx_op* op, double tol, long long max_iter, do
     long long outer = 0, sloppy_iters = 0;
     double res = hs.h->res;
     const int chunk = persistent_chunk(op->pat.nnz);
+    auto valsT_of = [&](auto& pcg) {
+        if constexpr (std::is_same<std::decay_t<decltype(*pcg.vals)>, float>::value)
+            return transposed(ctx, op, op->vals32, op->vals32T);
+        else
+            return transposed_values(ctx, op);
+    };
     auto run = [&](auto& pcg) -> int {
-        const int stt = pcg.brick            ? pcg.iterate_brick(chunk)
-                        : graph || pcg.hex ? pcg.iterate(check_every)
-                                           : pcg.iterate_persistent(chunk);
+        if (pcg.brick) return pcg.iterate_brick(chunk);
+        if (graph || pcg.hex) return pcg.iterate(check_every);
+        // solids: the shared-memory kernel's three-barrier form, which takes
+        // and leaves p as the kernel below does (an FP64 iteration of the mixed
+        // form at 80 x 16 x 16 19.7 -> 12.4 us; 160 x 16 x 16 has bricks)
+        int stt = -1;
+        if (op->ndof == 3 && ctx->pcg_smem)
+            stt = pcg.iterate_smem(chunk, valsT_of(pcg), 0);
+        if (stt < 0) stt = pcg.iterate_persistent(chunk);
         if (stt < 0)
             throw ModelFail{SVX_CUDA_ERROR, 0, -1,
                             "mixed precision below 50M nonzeros needs a cooperative launch"};
