@@ -342,12 +342,44 @@ void parallel_for(int32_t count, F&& fn) {
 }
 
 template <class T>
-void upload(svx_ctx* ctx, DBuf<T>& dst, const T* src, size_t count) {
+void upload_to(svx_ctx* ctx, DBuf<T>& dst, const T* src, size_t count) {
     dst.alloc(ctx->pool, count + 1);
     if (count)
         SVX_CUDA(cudaMemcpyAsync(dst.p, src, count * sizeof(T), cudaMemcpyHostToDevice,
                                  ctx->stream));
 }
+
+// Host bytes of a flat model's arrays that the device takes.
+size_t flat_bytes(const svx_flat_model_t* m, int64_t n_elem) {
+    const size_t nn = size_t(m->n_nodes), ne = size_t(n_elem);
+    return 24 * nn + 8 * nn * size_t(m->ndof) + 25 * ne + 8 +
+           4 * size_t(ne ? m->conn_ptr[ne] : 0) + 8 * size_t(m->n_fixed) + 16 * 10;
+}
+
+// Largest model (bytes) that is copied through the page-locked buffer.
+constexpr size_t STAGE_MAX = size_t(256) << 20;
+
+// Uploads through the context's staging buffer, which must be idle (every call
+// that used it has waited for its stream) and holds them until the next wait;
+// without room (bytes = 0) the copies run from the caller's memory.
+class Stager {
+public:
+    Stager(svx_ctx* ctx, size_t bytes)
+        : ctx_(ctx), at_(bytes ? static_cast<char*>(ctx->staging.get(bytes)) : nullptr) {}
+    template <class T>
+    void upload(DBuf<T>& dst, const T* src, size_t count) {
+        if (at_ && count) {
+            std::memcpy(at_, src, count * sizeof(T));
+            src = reinterpret_cast<const T*>(at_);
+            at_ += (count * sizeof(T) + 15) & ~size_t(15);
+        }
+        upload_to(ctx_, dst, src, count);
+    }
+
+private:
+    svx_ctx* ctx_;
+    char* at_;
+};
 
 float elapsed_ms(cudaEvent_t a, cudaEvent_t b) {
     float ms = 0.f;
@@ -392,15 +424,34 @@ void device_assemble(svx_ctx* ctx, svx_op* op) {
     SVX_CUDA(cudaEventRecord(ctx->ev[2], st));
     DBuf<double> ke;
     ke.alloc(ctx->pool, size_t(op->n_elem) * op->pat.ke_stride + 1);
-    uint64_t g = integrate_elements(ctx, op, ke.p, op->pat.ke_stride);
-    if (g != ~uint64_t(0)) {
-        int64_t g_fail = int64_t(g >> 8);
-        int g_reason = int(g & 0xff);
+    // the element kernel's verdict comes back with the pattern's sizes: one wait
+    DBuf<unsigned long long> fail;
+    fail.alloc(ctx->pool, 1);
+    integrate_elements_async(ctx, op, ke.p, op->pat.ke_stride, fail.p);
+    auto* h_fail = reinterpret_cast<unsigned long long*>(static_cast<char*>(ctx->h_scalars) +
+                                                         svx_ctx::H_FAIL);
+    SVX_CUDA(cudaMemcpyAsync(h_fail, fail.p, sizeof(*h_fail), cudaMemcpyDeviceToHost, st));
+    auto check_elements = [&]() {
+        const uint64_t g = *h_fail;
+        if (g == ~uint64_t(0)) return;
+        const int64_t g_fail = int64_t(g >> 8);
+        const int g_reason = int(g & 0xff);
         throw ModelFail{SVX_INVALID_MODEL, g_reason, g_fail,
                         "element " + std::to_string(op->h_elem_id[g_fail]) + ": " +
                             reason_text(g_reason)};
+    };
+    if (op->pat.row_ptr.p) {
+        SVX_CUDA(cudaStreamSynchronize(st));
+    } else {
+        try {
+            build_pattern(ctx, op);
+        } catch (const ModelFail&) {  // a bad element is reported before the pattern's limits
+            SVX_CUDA(cudaStreamSynchronize(st));
+            check_elements();
+            throw;
+        }
     }
-    if (!op->pat.row_ptr.p) build_pattern(ctx, op);
+    check_elements();
     op->vals.alloc(ctx->pool, op->pat.nnz + 1);
     assemble_values(ctx, op, ke.p, op->pat.ke_stride, op->vals.p);
     ke.reset();
@@ -417,6 +468,7 @@ void device_assemble(svx_ctx* ctx, svx_op* op) {
     op->spmv_group = choose_spmv_group(op);
     SVX_CUDA(cudaEventRecord(ctx->ev[3], st));
     op->ms_assemble = elapsed_ms(ctx->ev[2], ctx->ev[3]);
+    jacobi_condition(ctx, op);
 }
 
 // K1-K4 for a validated flat model; throws ModelFail for element errors.
@@ -463,13 +515,30 @@ svx_op* assemble_impl(svx_ctx* ctx, const svx_flat_model_t* m, uint32_t flags,
     op->flags = flags;
     cudaStream_t st = ctx->stream;
     SVX_CUDA(cudaEventRecord(ctx->ev[6], st));
-    upload(ctx, op->xyz, m->xyz, size_t(3 * m->n_nodes));
-    upload(ctx, op->kind, m->kind, size_t(op->n_elem));
-    upload(ctx, op->conn_ptr, m->conn_ptr, size_t(op->n_elem + 1));
-    upload(ctx, op->conn, m->conn, size_t(op->n_elem > 0 ? m->conn_ptr[op->n_elem] : 0));
-    upload(ctx, op->youngs, m->youngs, size_t(op->n_elem));
-    upload(ctx, op->poisson, m->poisson, size_t(op->n_elem));
-    if (thick_elem) upload(ctx, op->thick_elem, thick_elem, size_t(op->n_elem));
+    op->n_conn = op->n_elem > 0 ? m->conn_ptr[op->n_elem] : 0;
+    // the distinct constrained rows and each constraint's place among them
+    op->n_fixed = m->n_fixed;
+    op->h_fixed_row.assign(m->fixed_row, m->fixed_row + m->n_fixed);
+    std::vector<int64_t> uniq(op->h_fixed_row);
+    std::sort(uniq.begin(), uniq.end());
+    uniq.erase(std::unique(uniq.begin(), uniq.end()), uniq.end());
+    op->n_fixed_rows = int64_t(uniq.size());
+    std::vector<int32_t> slot(size_t(m->n_fixed));
+    for (int64_t k = 0; k < m->n_fixed; ++k)
+        slot[k] = int32_t(std::lower_bound(uniq.begin(), uniq.end(), op->h_fixed_row[k]) -
+                          uniq.begin());
+    // the caller's arrays go through the page-locked staging buffer (a copy
+    // from pageable memory waits for the stream each time); a batch's are in
+    // it already, and a model too large for it is copied as it lies
+    const bool staged = !prechecked && flat_bytes(m, op->n_elem) <= STAGE_MAX;
+    Stager stage(ctx, staged ? flat_bytes(m, op->n_elem) + 12 * size_t(m->n_fixed) + 1024 : 0);
+    stage.upload(op->xyz, m->xyz, size_t(3 * m->n_nodes));
+    stage.upload(op->kind, m->kind, size_t(op->n_elem));
+    stage.upload(op->conn_ptr, m->conn_ptr, size_t(op->n_elem + 1));
+    stage.upload(op->conn, m->conn, size_t(op->n_conn));
+    stage.upload(op->youngs, m->youngs, size_t(op->n_elem));
+    stage.upload(op->poisson, m->poisson, size_t(op->n_elem));
+    if (thick_elem) upload_to(ctx, op->thick_elem, thick_elem, size_t(op->n_elem));
     int max_nn = 0;
     op->all_hex = op->n_elem > 0;
     for (int64_t e = 0; e < op->n_elem; ++e) {
@@ -496,14 +565,14 @@ svx_op* assemble_impl(svx_ctx* ctx, const svx_flat_model_t* m, uint32_t flags,
     }
     // loads and constraints
     if (m->f) {
-        upload(ctx, op->f_orig, m->f, size_t(op->n));
+        stage.upload(op->f_orig, m->f, size_t(op->n));
     } else {
         op->f_orig.alloc(ctx->pool, size_t(op->n) + 1);
         SVX_CUDA(cudaMemsetAsync(op->f_orig.p, 0, sizeof(double) * size_t(op->n), st));
     }
-    op->n_fixed = m->n_fixed;
-    op->h_fixed_row.assign(m->fixed_row, m->fixed_row + m->n_fixed);
-    upload(ctx, op->fixed_row, op->h_fixed_row.data(), size_t(m->n_fixed));
+    stage.upload(op->fixed_row, op->h_fixed_row.data(), size_t(m->n_fixed));
+    stage.upload(op->fixed_uniq, uniq.data(), uniq.size());
+    stage.upload(op->fixed_slot, slot.data(), slot.size());
     op->h_node_id.resize(size_t(m->n_nodes));
     for (int64_t i = 0; i < m->n_nodes; ++i)
         op->h_node_id[i] = m->node_id ? m->node_id[i] : uint32_t(i + 1);
@@ -543,10 +612,11 @@ svx_op* assemble_mass_impl(svx_ctx* ctx, const svx_flat_model_t* m, double rho) 
     op->mass_rho = rho;
     cudaStream_t st = ctx->stream;
     SVX_CUDA(cudaEventRecord(ctx->ev[6], st));
-    upload(ctx, op->xyz, m->xyz, size_t(3 * m->n_nodes));
-    upload(ctx, op->kind, m->kind, size_t(op->n_elem));
-    upload(ctx, op->conn_ptr, m->conn_ptr, size_t(op->n_elem + 1));
-    upload(ctx, op->conn, m->conn, size_t(op->n_elem > 0 ? m->conn_ptr[op->n_elem] : 0));
+    upload_to(ctx, op->xyz, m->xyz, size_t(3 * m->n_nodes));
+    upload_to(ctx, op->kind, m->kind, size_t(op->n_elem));
+    upload_to(ctx, op->conn_ptr, m->conn_ptr, size_t(op->n_elem + 1));
+    op->n_conn = op->n_elem > 0 ? m->conn_ptr[op->n_elem] : 0;
+    upload_to(ctx, op->conn, m->conn, size_t(op->n_conn));
     int max_nn = 0;
     for (int64_t e = 0; e < op->n_elem; ++e) max_nn = std::max(max_nn, node_count(m->kind[e]));
     op->pat.max_nn = std::max(max_nn, 1);
@@ -578,20 +648,48 @@ void stress_to_device(svx_op* op) {
     recover_stress(ctx, op, op->u.p, op->vm_elem.p, op->vm_node.p, op->react.p, op->disp3.p);
 }
 
-void copy_stress_out(svx_op* op, svx_solution_t* sol) {
-    cudaStream_t st = op->ctx->stream;
-    if (sol->von_mises && op->n_elem)
-        SVX_CUDA(cudaMemcpyAsync(sol->von_mises, op->vm_elem.p, op->n_elem * sizeof(double),
-                                 cudaMemcpyDeviceToHost, st));
-    if (sol->nodal_von_mises && op->n_nodes)
-        SVX_CUDA(cudaMemcpyAsync(sol->nodal_von_mises, op->vm_node.p,
-                                 op->n_nodes * sizeof(double), cudaMemcpyDeviceToHost, st));
-    if (sol->reactions && op->n_fixed)
-        SVX_CUDA(cudaMemcpyAsync(sol->reactions, op->react.p, op->n_fixed * sizeof(double),
-                                 cudaMemcpyDeviceToHost, st));
-    if (sol->displacements && op->n_nodes)
-        SVX_CUDA(cudaMemcpyAsync(sol->displacements, op->disp3.p,
-                                 3 * op->n_nodes * sizeof(double), cudaMemcpyDeviceToHost, st));
+// Results to the caller's arrays: through the idle staging buffer, so that the
+// copies run as DMA behind one another, and from there after the wait
+// (finish()); sets too large for it are copied as they lie.
+class Fetcher {
+public:
+    Fetcher(svx_ctx* ctx, size_t bytes)
+        : ctx_(ctx),
+          at_(bytes <= STAGE_MAX ? static_cast<char*>(ctx->staging.get(bytes + 1024)) : nullptr) {}
+    void add(double* to, const double* from, int64_t count) {
+        if (!to || count <= 0) return;
+        const size_t bytes = size_t(count) * sizeof(double);
+        double* via = at_ ? reinterpret_cast<double*>(at_) : to;
+        SVX_CUDA(cudaMemcpyAsync(via, from, bytes, cudaMemcpyDeviceToHost, ctx_->stream));
+        if (!at_) return;
+        parts_.push_back({to, via, bytes});
+        at_ += (bytes + 15) & ~size_t(15);
+    }
+    void finish() {
+        SVX_CUDA(cudaStreamSynchronize(ctx_->stream));
+        for (const Part& p : parts_) std::memcpy(p.to, p.via, p.bytes);
+        parts_.clear();
+    }
+
+private:
+    struct Part {
+        double *to, *via;
+        size_t bytes;
+    };
+    svx_ctx* ctx_;
+    char* at_;
+    std::vector<Part> parts_;
+};
+
+size_t solution_bytes(const svx_op* op) {
+    return 8 * size_t(op->n + op->n_elem + 4 * op->n_nodes + op->n_fixed);
+}
+
+void copy_stress_out(svx_op* op, const svx_solution_t* sol, Fetcher& out) {
+    out.add(sol->von_mises, op->vm_elem.p, op->n_elem);
+    out.add(sol->nodal_von_mises, op->vm_node.p, op->n_nodes);
+    out.add(sol->reactions, op->react.p, op->n_fixed);
+    out.add(sol->displacements, op->disp3.p, 3 * op->n_nodes);
 }
 
 long long default_max_iter(int64_t n) { return std::max<long long>(1000, 10 * (long long)n); }
@@ -633,6 +731,7 @@ int solve_impl(svx_op* op, const svx_solve_opts_t* o, svx_solution_t* sol, svx_e
         outer = 0;
     }
     op->has_solution = true;
+    Fetcher out(ctx, sol ? solution_bytes(op) : 0);
     if (sol) {
         sol->iterations = r.iterations;
         sol->outer_iterations = outer;
@@ -645,12 +744,10 @@ int solve_impl(svx_op* op, const svx_solve_opts_t* o, svx_solution_t* sol, svx_e
         sol->ms_factor = direct ? dres.ms : 0.0;
         sol->ms_assemble = op->ms_assemble;
         sol->ms_solve = r.ms;
-        if (sol->u)
-            SVX_CUDA(cudaMemcpyAsync(sol->u, op->u.p, op->n * sizeof(double),
-                                     cudaMemcpyDeviceToHost, ctx->stream));
+        out.add(sol->u, op->u.p, op->n);
     }
     if (r.status != PCG_CONVERGED) {
-        SVX_CUDA(cudaStreamSynchronize(ctx->stream));
+        out.finish();
         std::string msg = "not converged after " + std::to_string(r.iterations) + " iterations";
         fill_error(err, SVX_NOT_CONVERGED, 0, -1, msg);
         if (err) {
@@ -665,11 +762,11 @@ int solve_impl(svx_op* op, const svx_solve_opts_t* o, svx_solution_t* sol, svx_e
         stress_to_device(op);
         SVX_CUDA(cudaEventRecord(ctx->ev[5], ctx->stream));
         if (sol) {
-            copy_stress_out(op, sol);
+            copy_stress_out(op, sol, out);
             sol->ms_stress = elapsed_ms(ctx->ev[4], ctx->ev[5]);
         }
     }
-    SVX_CUDA(cudaStreamSynchronize(ctx->stream));
+    out.finish();
     clear_error(err);
     return SVX_OK;
 }
@@ -1207,12 +1304,11 @@ int svx_op_stress(svx_op_t* op, svx_solution_t* sol) {
         SVX_CUDA(cudaEventRecord(ctx->ev[4], st));
         stress_to_device(op);
         SVX_CUDA(cudaEventRecord(ctx->ev[5], st));
-        copy_stress_out(op, sol);
-        if (sol->u)
-            SVX_CUDA(cudaMemcpyAsync(sol->u, op->u.p, op->n * sizeof(double),
-                                     cudaMemcpyDeviceToHost, st));
+        Fetcher out(ctx, solution_bytes(op));
+        copy_stress_out(op, sol, out);
+        out.add(sol->u, op->u.p, op->n);
         sol->ms_stress = elapsed_ms(ctx->ev[4], ctx->ev[5]);
-        SVX_CUDA(cudaStreamSynchronize(st));
+        out.finish();
         return SVX_OK;
     });
 }
@@ -1339,10 +1435,11 @@ int svx_solve_thermal_flat(svx_ctx_t* ctx, const svx_thermal_model_t* m,
         op->thickness = m->thickness;
         cudaStream_t st = ctx->stream;
         SVX_CUDA(cudaEventRecord(ctx->ev[6], st));
-        upload(ctx, op->xyz, m->xyz, size_t(3 * m->n_nodes));
-        upload(ctx, op->kind, m->kind, size_t(m->n_elem));
-        upload(ctx, op->conn_ptr, m->conn_ptr, size_t(m->n_elem + 1));
-        upload(ctx, op->conn, m->conn, size_t(m->conn_ptr[m->n_elem]));
+        upload_to(ctx, op->xyz, m->xyz, size_t(3 * m->n_nodes));
+        upload_to(ctx, op->kind, m->kind, size_t(m->n_elem));
+        upload_to(ctx, op->conn_ptr, m->conn_ptr, size_t(m->n_elem + 1));
+        op->n_conn = m->conn_ptr[m->n_elem];
+        upload_to(ctx, op->conn, m->conn, size_t(op->n_conn));
         op->pat.max_nn = max_nn;
         op->pat.ke_stride = max_nn * max_nn;
         DBuf<double> ke, fe;
@@ -1389,9 +1486,9 @@ int svx_solve_thermal_flat(svx_ctx_t* ctx, const svx_thermal_model_t* m,
         DBuf<int32_t> d_face;
         DBuf<double> d_flux;
         if (m->n_flux > 0) {
-            upload(ctx, d_fe_elem, m->flux_elem, size_t(m->n_flux));
-            upload(ctx, d_face, m->flux_face, size_t(m->n_flux));
-            upload(ctx, d_flux, m->flux_value, size_t(m->n_flux));
+            upload_to(ctx, d_fe_elem, m->flux_elem, size_t(m->n_flux));
+            upload_to(ctx, d_face, m->flux_face, size_t(m->n_flux));
+            upload_to(ctx, d_flux, m->flux_value, size_t(m->n_flux));
         }
         op->f.alloc(ctx->pool, size_t(op->n) + 1);
         thermal_loads(ctx, op.get(), fe.p, m->has_source, m->n_flux, d_fe_elem.p, d_face.p,
@@ -1401,7 +1498,7 @@ int svx_solve_thermal_flat(svx_ctx_t* ctx, const svx_thermal_model_t* m,
         std::vector<double> pres(size_t(op->n), std::nan(""));
         for (int64_t q = 0; q < m->n_temp; ++q) pres[m->temp_node[q]] = m->temp_value[q];
         DBuf<double> d_pres;
-        upload(ctx, d_pres, pres.data(), pres.size());
+        upload_to(ctx, d_pres, pres.data(), pres.size());
         apply_temperatures(ctx, op.get(), d_pres.p);
         jacobi_diagonal(ctx, op.get());
         SVX_CUDA(cudaEventRecord(ctx->ev[7], st));

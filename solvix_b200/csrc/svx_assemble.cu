@@ -92,10 +92,29 @@ __global__ void mark_fixed_kernel(int64_t n_fixed, const int64_t* __restrict__ r
 }
 
 // Row lengths of the compact constrained rows.
-__global__ void fixed_len_kernel(int64_t m, const int64_t* __restrict__ rows,
-                                 const int32_t* __restrict__ row_ptr, int32_t* __restrict__ len) {
-    int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k < m) len[k] = row_ptr[rows[k] + 1] - row_ptr[rows[k]];
+// ptr[0..m]: exclusive sums of the rows' lengths; one block.
+__global__ void __launch_bounds__(1024)
+fixed_ptr_kernel(int64_t m, const int64_t* __restrict__ rows, const int32_t* __restrict__ row_ptr,
+                 int32_t* __restrict__ ptr) {
+    __shared__ int32_t sums[1024];
+    const int t = threadIdx.x;
+    const int64_t per = (m + 1023) / 1024, k0 = min(m, per * t), k1 = min(m, k0 + per);
+    int32_t own = 0;
+    for (int64_t k = k0; k < k1; ++k) own += row_ptr[rows[k] + 1] - row_ptr[rows[k]];
+    sums[t] = own;
+    __syncthreads();
+    for (int off = 1; off < 1024; off <<= 1) {
+        const int32_t v = t >= off ? sums[t - off] : 0;
+        __syncthreads();
+        sums[t] += v;
+        __syncthreads();
+    }
+    int32_t at = sums[t] - own;
+    for (int64_t k = k0; k < k1; ++k) {
+        ptr[k] = at;
+        at += row_ptr[rows[k] + 1] - row_ptr[rows[k]];
+    }
+    if (t == 1023) ptr[m] = sums[1023];
 }
 
 // Copy the unmodified constrained rows (one warp per row).
@@ -163,6 +182,32 @@ __global__ void diag_kernel(int64_t n, const int32_t* __restrict__ diag_pos,
     }
 }
 
+// out[0], out[1]: the largest and the smallest of the blocks' extremes (0 and
+// infinity without blocks).
+__global__ void __launch_bounds__(256)
+extremes_kernel(int64_t nb, const double* hi, const double* lo, double* out) {
+    __shared__ double shi[256], slo[256];
+    double h = 0.0, l = INFINITY;
+    for (int64_t k = threadIdx.x; k < nb; k += 256) {
+        h = fmax(h, hi[k]);
+        l = fmin(l, lo[k]);
+    }
+    shi[threadIdx.x] = h;
+    slo[threadIdx.x] = l;
+    __syncthreads();
+    for (int off = 128; off > 0; off >>= 1) {
+        if (threadIdx.x < off) {
+            shi[threadIdx.x] = fmax(shi[threadIdx.x], shi[threadIdx.x + off]);
+            slo[threadIdx.x] = fmin(slo[threadIdx.x], slo[threadIdx.x + off]);
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        out[0] = shi[0];
+        out[1] = slo[0];
+    }
+}
+
 inline unsigned blocks_for(int64_t n, int t) { return unsigned((n + t - 1) / t); }
 
 }  // namespace
@@ -200,43 +245,29 @@ void apply_dirichlet(svx_ctx* ctx, svx_op* op) {
             op->n_fixed, op->fixed_row.p, op->is_fixed.p);
         SVX_LAUNCH_CHECK();
     }
-    // compact copy of the constrained rows of the unmodified K
-    std::vector<int64_t> uniq(op->h_fixed_row);
-    std::sort(uniq.begin(), uniq.end());
-    uniq.erase(std::unique(uniq.begin(), uniq.end()), uniq.end());
-    const int64_t m = int64_t(uniq.size());
-    op->n_fixed_rows = m;
-    std::vector<int32_t> slot(op->n_fixed);
-    for (int64_t k = 0; k < op->n_fixed; ++k)
-        slot[k] = int32_t(std::lower_bound(uniq.begin(), uniq.end(), op->h_fixed_row[k]) -
-                          uniq.begin());
-    op->fixed_slot.alloc(ctx->pool, op->n_fixed + 1);
-    op->kc_ptr.alloc(ctx->pool, m + 1);
+    // compact copy of the constrained rows of the unmodified K (fixed_uniq and
+    // fixed_slot were uploaded with the model)
+    const int64_t m = op->n_fixed_rows;
     if (m > 0) {
-        DBuf<int64_t> d_uniq;
-        DBuf<int32_t> d_len;
-        d_uniq.alloc(ctx->pool, m);
-        d_len.alloc(ctx->pool, m);
-        SVX_CUDA(cudaMemcpyAsync(d_uniq.p, uniq.data(), m * sizeof(int64_t),
-                                 cudaMemcpyHostToDevice, st));
-        SVX_CUDA(cudaMemcpyAsync(op->fixed_slot.p, slot.data(), op->n_fixed * sizeof(int32_t),
-                                 cudaMemcpyHostToDevice, st));
-        fixed_len_kernel<<<blocks_for(m, 256), 256, 0, st>>>(m, d_uniq.p, P.row_ptr.p, d_len.p);
+        op->kc_ptr.alloc(ctx->pool, m + 1);
+        fixed_ptr_kernel<<<1, 1024, 0, st>>>(m, op->fixed_uniq.p, P.row_ptr.p, op->kc_ptr.p);
         SVX_LAUNCH_CHECK();
-        std::vector<int32_t> len(m), ptr(m + 1, 0);
-        SVX_CUDA(cudaMemcpyAsync(len.data(), d_len.p, m * sizeof(int32_t),
-                                 cudaMemcpyDeviceToHost, st));
-        SVX_CUDA(cudaStreamSynchronize(st));
-        for (int64_t k = 0; k < m; ++k) ptr[k + 1] = ptr[k] + len[k];
-        SVX_CUDA(cudaMemcpyAsync(op->kc_ptr.p, ptr.data(), (m + 1) * sizeof(int32_t),
-                                 cudaMemcpyHostToDevice, st));
-        op->kc_col.alloc(ctx->pool, size_t(ptr[m]) + 1);
-        op->kc_val.alloc(ctx->pool, size_t(ptr[m]) + 1);
+        // room for every row at the largest degree, where that is small, saves
+        // the wait for the rows' own total
+        int64_t room = m * int64_t(op->ndof) * std::max(1, P.max_deg);
+        if (room > (int64_t(1) << 26)) {
+            int32_t total = 0;
+            SVX_CUDA(cudaMemcpyAsync(&total, op->kc_ptr.p + m, sizeof(total),
+                                     cudaMemcpyDeviceToHost, st));
+            SVX_CUDA(cudaStreamSynchronize(st));
+            room = total;
+        }
+        op->kc_col.alloc(ctx->pool, size_t(room) + 1);
+        op->kc_val.alloc(ctx->pool, size_t(room) + 1);
         fixed_copy_kernel<<<blocks_for(m * 32, 256), 256, 0, st>>>(
-            m, d_uniq.p, P.row_ptr.p, P.col_idx.p, op->vals.p, op->kc_ptr.p, op->kc_col.p,
-            op->kc_val.p);
+            m, op->fixed_uniq.p, P.row_ptr.p, P.col_idx.p, op->vals.p, op->kc_ptr.p,
+            op->kc_col.p, op->kc_val.p);
         SVX_LAUNCH_CHECK();
-        SVX_CUDA(cudaStreamSynchronize(st));
     }
     // f_orig keeps the unmodified loads; f gets the eliminated copy
     op->f.alloc(ctx->pool, n + 1);
@@ -259,26 +290,22 @@ void jacobi_diagonal(svx_ctx* ctx, svx_op* op) {
     const int64_t nb = (n + 255) / 256;
     DBuf<double> bhi, blo;
     bhi.alloc(ctx->pool, nb + 1);
-    blo.alloc(ctx->pool, nb + 1);
+    blo.alloc(ctx->pool, nb + 2);  // and the extremes of all blocks
     if (n > 0) {
         diag_kernel<<<unsigned(nb), 256, 0, st>>>(n, P.diag_pos.p, op->vals.p, op->inv_diag.p,
                                                   bhi.p, blo.p);
         SVX_LAUNCH_CHECK();
     }
-    std::vector<double> hhi(nb), hlo(nb);
-    if (nb > 0) {
-        SVX_CUDA(cudaMemcpyAsync(hhi.data(), bhi.p, nb * sizeof(double), cudaMemcpyDeviceToHost,
-                                 st));
-        SVX_CUDA(cudaMemcpyAsync(hlo.data(), blo.p, nb * sizeof(double), cudaMemcpyDeviceToHost,
-                                 st));
-    }
-    SVX_CUDA(cudaStreamSynchronize(st));
-    double hi = 0.0, lo = INFINITY;
-    for (int64_t b = 0; b < nb; ++b) {
-        hi = std::fmax(hi, hhi[b]);
-        lo = std::fmin(lo, hlo[b]);
-    }
-    op->cond_estimate = hi / lo;
+    double* h = reinterpret_cast<double*>(static_cast<char*>(ctx->h_scalars) + svx_ctx::H_DIAG);
+    extremes_kernel<<<1, 256, 0, st>>>(nb, bhi.p, blo.p, blo.p + nb);
+    SVX_LAUNCH_CHECK();
+    SVX_CUDA(cudaMemcpyAsync(h, blo.p + nb, 2 * sizeof(double), cudaMemcpyDeviceToHost, st));
+}
+
+void jacobi_condition(svx_ctx* ctx, svx_op* op) {
+    const double* h = reinterpret_cast<const double*>(static_cast<const char*>(ctx->h_scalars) +
+                                                      svx_ctx::H_DIAG);
+    op->cond_estimate = h[0] / h[1];
 }
 
 }  // namespace svx

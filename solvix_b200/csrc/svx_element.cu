@@ -999,19 +999,24 @@ inline unsigned blocks_for(int64_t n, int t) { return unsigned((n + t - 1) / t);
 
 }  // namespace
 
-uint64_t integrate_elements(svx_ctx* ctx, svx_op* op, double* ke, int ke_stride) {
-    DBuf<unsigned long long> fail;
-    fail.alloc(ctx->pool, 1);
-    SVX_CUDA(cudaMemsetAsync(fail.p, 0xff, sizeof(unsigned long long), ctx->stream));
+void integrate_elements_async(svx_ctx* ctx, svx_op* op, double* ke, int ke_stride,
+                              unsigned long long* fail) {
+    SVX_CUDA(cudaMemsetAsync(fail, 0xff, sizeof(unsigned long long), ctx->stream));
     if (op->n_elem > 0) {
         int64_t blocks = (op->n_elem + WARPS - 1) / WARPS;
         int64_t cap = int64_t(ctx->sm_count) * 64;
         if (blocks > cap) blocks = cap;
         integrate_kernel<<<unsigned(blocks), WARPS * 32, 0, ctx->stream>>>(
             op->n_elem, op->kind.p, op->conn_ptr.p, op->conn.p, op->xyz.p, op->youngs.p,
-            op->poisson.p, op->thickness, op->thick_elem.p, ke, ke_stride, fail.p);
+            op->poisson.p, op->thickness, op->thick_elem.p, ke, ke_stride, fail);
         SVX_LAUNCH_CHECK();
     }
+}
+
+uint64_t integrate_elements(svx_ctx* ctx, svx_op* op, double* ke, int ke_stride) {
+    DBuf<unsigned long long> fail;
+    fail.alloc(ctx->pool, 1);
+    integrate_elements_async(ctx, op, ke, ke_stride, fail.p);
     unsigned long long h = 0;
     SVX_CUDA(cudaMemcpyAsync(&h, fail.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     SVX_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1042,7 +1047,7 @@ void recover_stress(svx_ctx* ctx, svx_op* op, const double* u, double* vm_elem, 
                 vm_node);
             SVX_LAUNCH_CHECK();
         }
-        SVX_CUDA(cudaStreamSynchronize(st));
+        // nodal goes back to the pool; its next user is behind this stream
     }
     if (reactions && op->n_fixed > 0) {
         reactions_kernel<<<blocks_for(op->n_fixed, 128), 128, 0, st>>>(

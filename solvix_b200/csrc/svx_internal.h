@@ -138,7 +138,8 @@ public:
             if (p_) cudaFreeHost(p_);
             p_ = nullptr;
             cap_ = 0;
-            const size_t want = std::max(bytes, cap_ + cap_ / 2);
+            size_t want = size_t(1) << 20;  // sizes double, so a growing series allocates rarely
+            while (want < bytes) want *= 2;
             cudaError_t e = cudaHostAlloc(&p_, want, cudaHostAllocDefault);
             if (e != cudaSuccess) {
                 cudaGetLastError();
@@ -173,6 +174,9 @@ struct svx_ctx {
     std::string last_error;
     cudaEvent_t ev[8] = {};
     void* h_scalars = nullptr;  // page-locked PcgScalars of the context's solves
+    // what the assembly reads back in it, byte offsets (the pattern's sizes are
+    // at 0): the element kernel's failure, the extreme diagonals
+    static constexpr int H_FAIL = 64, H_DIAG = 96;
     // largest per-block shared-memory adjacency of the persistent PCG kernels
     // (bytes; 0 keeps it in global memory); SVX_SHARED_ADJ_MAX in the
     // environment at svx_ctx_create overrides the build's default
@@ -332,6 +336,7 @@ struct svx_op {
     svx::DBuf<uint8_t> kind;
     svx::DBuf<int64_t> conn_ptr;
     svx::DBuf<int32_t> conn;
+    int64_t n_conn = 0;  // its entries
     svx::DBuf<double> youngs, poisson;
     svx::DBuf<double> thick_elem;  // per-element thickness (batched models), else empty
     // the chip-resident PCG's node order (svx_resident.cu): per member, slot
@@ -365,6 +370,7 @@ struct svx_op {
     int64_t n_fixed = 0;
     int64_t n_fixed_rows = 0;
     svx::DBuf<int64_t> fixed_row;      // [n_fixed] BC order
+    svx::DBuf<int64_t> fixed_uniq;     // [n_fixed_rows] the distinct rows, ascending
     svx::DBuf<int32_t> fixed_slot;     // [n_fixed] -> compact row
     svx::DBuf<int32_t> kc_ptr;         // [n_fixed_rows + 1]
     svx::DBuf<int32_t> kc_col;
@@ -401,12 +407,17 @@ void build_pattern(svx_ctx* ctx, svx_op* op);
 // Element integration into a Ke buffer; returns the first failing element
 // as (index << 8 | reason) or UINT64_MAX (svx_element.cu).
 uint64_t integrate_elements(svx_ctx* ctx, svx_op* op, double* ke, int ke_stride);
+// The same without the wait: fail (device, one value) gets what it returns.
+void integrate_elements_async(svx_ctx* ctx, svx_op* op, double* ke, int ke_stride,
+                              unsigned long long* fail);
 // Fixed-order gather of Ke into CSR values (svx_assemble.cu).
 void assemble_values(svx_ctx* ctx, svx_op* op, const double* ke, int ke_stride, double* vals);
 // Dirichlet + inverse diagonal + condition estimate (svx_assemble.cu).
 void apply_dirichlet(svx_ctx* ctx, svx_op* op);
-// Inverse diagonal and condition estimate of op->vals alone (svx_assemble.cu).
+// Inverse diagonal and condition estimate of op->vals alone (svx_assemble.cu);
+// jacobi_condition reads the estimate once the stream has been waited for.
 void jacobi_diagonal(svx_ctx* ctx, svx_op* op);
+void jacobi_condition(svx_ctx* ctx, svx_op* op);
 // The graph form's FP32 difference-form SpMV with p.q, for FP64 (V =
 // double) or FP32 (V = float) vectors (svx_pcg.cu); at most `grid` blocks.
 template <class V>
@@ -557,7 +568,6 @@ void run_batch(svx_ctx* ctx, int32_t count, const svx_flat_model_t* const* model
                std::vector<BatchModelOut>& out, BatchRun& run);
 
 // Generic device helpers (svx_pattern.cu).
-void exclusive_scan_i64(svx_ctx* ctx, const int64_t* in, int64_t* out, int64_t n,
-                        int64_t* total_host);
+void exclusive_scan_i64(svx_ctx* ctx, const int64_t* in, int64_t* out, int64_t n);
 
 }  // namespace svx

@@ -83,8 +83,8 @@ void scan_rec(svx_ctx* ctx, const int64_t* in, int64_t* out, int64_t n) {
         scan_add_kernel<<<unsigned((n + 255) / 256), 256, 0, ctx->stream>>>(out, n, offs.p);
         SVX_LAUNCH_CHECK();
     }
-    // keep the temporaries alive until the stream has consumed them
-    SVX_CUDA(cudaStreamSynchronize(ctx->stream));
+    // the temporaries go back to the context's pool, whose later users are
+    // ordered behind this stream
 }
 
 // ---- 1. incidence ---------------------------------------------------------
@@ -259,16 +259,11 @@ inline unsigned blocks_for(int64_t n, int t) { return unsigned((n + t - 1) / t);
 
 }  // namespace
 
-void exclusive_scan_i64(svx_ctx* ctx, const int64_t* in, int64_t* out, int64_t n,
-                        int64_t* total_host) {
+// out[0..n]: exclusive sums of in and their total, all on the device.
+void exclusive_scan_i64(svx_ctx* ctx, const int64_t* in, int64_t* out, int64_t n) {
     scan_rec(ctx, in, out, n);
     scan_total_kernel<<<1, 1, 0, ctx->stream>>>(in, out, n);
     SVX_LAUNCH_CHECK();
-    if (total_host) {
-        SVX_CUDA(cudaMemcpyAsync(total_host, out + n, sizeof(int64_t), cudaMemcpyDeviceToHost,
-                                 ctx->stream));
-        SVX_CUDA(cudaStreamSynchronize(ctx->stream));
-    }
 }
 
 void build_pattern(svx_ctx* ctx, svx_op* op) {
@@ -296,8 +291,8 @@ void build_pattern(svx_ctx* ctx, svx_op* op) {
         SVX_LAUNCH_CHECK();
     }
     P.slot_ptr.alloc(ctx->pool, nn + 1);
-    int64_t n_slots = 0;
-    exclusive_scan_i64(ctx, cnt.p, P.slot_ptr.p, nn, &n_slots);
+    exclusive_scan_i64(ctx, cnt.p, P.slot_ptr.p, nn);
+    const int64_t n_slots = op->n_conn;
     P.n_slots = n_slots;
     keys.alloc(ctx->pool, n_slots + 1);
     P.slot_elem.alloc(ctx->pool, n_slots + 1);
@@ -327,17 +322,9 @@ void build_pattern(svx_ctx* ctx, svx_op* op) {
         SVX_LAUNCH_CHECK();
     }
     P.adj_ptr.alloc(ctx->pool, nn + 1);
-    int64_t n_adj = 0;
-    exclusive_scan_i64(ctx, deg.p, P.adj_ptr.p, nn, &n_adj);
-    P.adj.alloc(ctx->pool, n_adj + 1);
-    if (nn > 0) {
-        adjacency_kernel<<<blocks_for(nn, 128), 128, 0, st>>>(
-            nn, P.slot_ptr.p, P.slot_elem.p, op->conn_ptr.p, op->conn.p, nullptr, P.adj_ptr.p,
-            P.adj.p, nullptr);
-        SVX_LAUNCH_CHECK();
-    }
+    exclusive_scan_i64(ctx, deg.p, P.adj_ptr.p, nn);
 
-    // 3. rows
+    // 3. rows, and the one wait of the pattern: the sizes that follow
     DBuf<int64_t> node_nnz;
     node_nnz.alloc(ctx->pool, nn + 1);
     if (nn > 0) {
@@ -346,12 +333,35 @@ void build_pattern(svx_ctx* ctx, svx_op* op) {
         SVX_LAUNCH_CHECK();
     }
     P.node_base.alloc(ctx->pool, nn + 1);
-    int64_t nnz = 0;
-    exclusive_scan_i64(ctx, node_nnz.p, P.node_base.p, nn, &nnz);
+    exclusive_scan_i64(ctx, node_nnz.p, P.node_base.p, nn);
+    struct Sizes {
+        int64_t n_adj, nnz;
+        int flags[2];
+    };
+    Sizes* h = static_cast<Sizes*>(ctx->h_scalars);
+    SVX_CUDA(cudaMemcpyAsync(&h->n_adj, P.adj_ptr.p + nn, sizeof(int64_t),
+                             cudaMemcpyDeviceToHost, st));
+    SVX_CUDA(cudaMemcpyAsync(&h->nnz, P.node_base.p + nn, sizeof(int64_t),
+                             cudaMemcpyDeviceToHost, st));
+    SVX_CUDA(cudaMemcpyAsync(h->flags, flags.p, sizeof(h->flags), cudaMemcpyDeviceToHost, st));
+    SVX_CUDA(cudaStreamSynchronize(st));
+    const int64_t n_adj = h->n_adj, nnz = h->nnz;
+    P.max_slots = h->flags[0];
+    P.max_deg = h->flags[1];
     if (nnz >= int64_t(INT_MAX))
         throw ModelFail{SVX_OOM, 0, -1,
                         "stiffness has " + std::to_string(nnz) +
                             " nonzeros; the int32 CSR indices of the device path hold < 2^31"};
+    if (P.max_deg > 65535)
+        throw ModelFail{SVX_INVALID_MODEL, 0, -1,
+                        "a node shares elements with more than 65535 nodes"};
+    P.adj.alloc(ctx->pool, n_adj + 1);
+    if (nn > 0) {
+        adjacency_kernel<<<blocks_for(nn, 128), 128, 0, st>>>(
+            nn, P.slot_ptr.p, P.slot_elem.p, op->conn_ptr.p, op->conn.p, nullptr, P.adj_ptr.p,
+            P.adj.p, nullptr);
+        SVX_LAUNCH_CHECK();
+    }
     P.nnz = nnz;
     P.row_ptr.alloc(ctx->pool, P.n + 1);
     P.col_idx.alloc(ctx->pool, nnz + 1);
@@ -371,14 +381,6 @@ void build_pattern(svx_ctx* ctx, svx_op* op) {
             P.adj.p, P.slot_map.p);
         SVX_LAUNCH_CHECK();
     }
-    int h_flags[2] = {0, 0};
-    SVX_CUDA(cudaMemcpyAsync(h_flags, flags.p, sizeof(h_flags), cudaMemcpyDeviceToHost, st));
-    SVX_CUDA(cudaStreamSynchronize(st));
-    P.max_slots = h_flags[0];
-    P.max_deg = h_flags[1];
-    if (P.max_deg > 65535)
-        throw ModelFail{SVX_INVALID_MODEL, 0, -1,
-                        "a node shares elements with more than 65535 nodes"};
 }
 
 }  // namespace svx
