@@ -30,57 +30,88 @@ namespace {
 
 constexpr int ASM_WARPS = 8;
 
+// The sums of one slot: rows (ND x NN ND) of the element's Ke onto the node's
+// block, the lanes of its group one value each.
+template <int ND, int NN, int G>
+__device__ __forceinline__ void add_rows(double* acc, int rowlen, const uint16_t* map,
+                                         const double* rows, int gl) {
+    constexpr int N = NN * ND;
+#pragma unroll
+    for (int t0 = 0; t0 < ND * N; t0 += G) {
+        const int t = t0 + gl;
+        if (ND * N % G != 0 && t >= ND * N) break;
+        const int da = t / N, col = t - da * N, c = col / ND, db = col - c * ND;
+        acc[da * rowlen + int(map[c]) * ND + db] += rows[t];
+    }
+}
+
+// G lanes a node: a warp for plane and solid rows, eight lanes for one dof a
+// node (an element's row is at most eight values then; a warp a node left 24
+// lanes idle: 899 us for the 240 x 24 x 24 conduction block, 92 now).  Whether an
+// element repeats a node is found by one match over its map (reading the map
+// pair by pair was most of this kernel's loads; with the sizes of an element
+// known at compile time the 160 x 16 x 16 solid assembles in 1.37 ms instead of
+// 1.56, the 40 solids of a batch in 8.2 instead of 9.7).
+template <int ND>
 __global__ void __launch_bounds__(ASM_WARPS * 32)
-assemble_kernel(int64_t n_nodes, int ndof, int max_nn, int acc_stride,
+assemble_kernel(int64_t n_nodes, int max_nn, int acc_stride,
                 const int64_t* __restrict__ slot_ptr, const int32_t* __restrict__ slot_elem,
                 const uint8_t* __restrict__ slot_local, const uint16_t* __restrict__ slot_map,
                 const int64_t* __restrict__ conn_ptr, const int64_t* __restrict__ adj_ptr,
                 const int64_t* __restrict__ node_base, const double* __restrict__ ke,
                 int ke_stride, double* __restrict__ vals) {
+    constexpr int G = ND == 1 ? 8 : 32, PER = 32 / G;
     extern __shared__ double acc_all[];
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1), grp = lane / G;
     const int w = threadIdx.x >> 5;
-    double* acc = acc_all + size_t(w) * acc_stride;
-    const int64_t warps_total = int64_t(gridDim.x) * ASM_WARPS;
-    for (int64_t i = int64_t(blockIdx.x) * ASM_WARPS + w; i < n_nodes; i += warps_total) {
-        const int64_t deg = adj_ptr[i + 1] - adj_ptr[i];
-        const int64_t base = node_base[i];
-        if (deg == 0) {  // unreferenced node: only the diagonal seeds
-            if (lane < ndof) vals[base + lane] = 0.0;
-            continue;
-        }
-        const int rowlen = int(ndof * deg);
-        const int total = ndof * rowlen;
-        for (int q = lane; q < total; q += 32) acc[q] = 0.0;
+    double* acc = acc_all + size_t(w * PER + grp) * acc_stride;
+    const int warps = int(blockDim.x) >> 5;
+    const int64_t step = int64_t(gridDim.x) * warps * PER;
+    for (int64_t i0 = (int64_t(blockIdx.x) * warps + w) * PER; i0 < n_nodes; i0 += step) {
+        const int64_t i = i0 + grp;
+        const bool node = i < n_nodes;
+        const int64_t deg = node ? adj_ptr[i + 1] - adj_ptr[i] : 0;
+        const int64_t base = node ? node_base[i] : 0;
+        if (node && deg == 0 && gl < ND) vals[base + gl] = 0.0;  // only the diagonal seeds
+        const int rowlen = int(ND * deg);
+        const int total = ND * rowlen;
+        for (int q = gl; q < total; q += G) acc[q] = 0.0;
+        const int64_t s0 = deg > 0 ? slot_ptr[i] : 0;
+        const int slots = deg > 0 ? int(slot_ptr[i + 1] - s0) : 0;
+        const int most = PER == 1 ? slots : __reduce_max_sync(0xffffffffu, slots);
         __syncwarp();
-        const int64_t s1 = slot_ptr[i + 1];
-        for (int64_t s = slot_ptr[i]; s < s1; ++s) {
-            const int64_t e = slot_elem[s];
-            const int a = slot_local[s];
-            const int nn = int(conn_ptr[e + 1] - conn_ptr[e]);
-            const int N = nn * ndof;
+        for (int k = 0; k < most; ++k) {
+            const bool on = k < slots;
+            const int64_t s = s0 + k;
+            const int64_t e = on ? slot_elem[s] : 0;
+            const int a = on ? slot_local[s] : 0;
+            const int nn = on ? int(conn_ptr[e + 1] - conn_ptr[e]) : 0;
+            const int N = nn * ND;
             const uint16_t* map = slot_map + s * max_nn;
-            const double* rows = ke + e * int64_t(ke_stride) + int64_t(a) * ndof * N;
+            const double* rows = ke + e * int64_t(ke_stride) + int64_t(a) * ND * N;
             // an element that repeats a node maps two columns to one target
-            bool dup = false;
-            for (int c = 0; c < nn; ++c)
-                for (int c2 = c + 1; c2 < nn; ++c2) dup |= (map[c] == map[c2]);
-            if (!dup) {
-                for (int t = lane; t < ndof * N; t += 32) {
-                    int da = t / N, col = t - da * N;
-                    int c = col / ndof, db = col - c * ndof;
-                    acc[da * rowlen + int(map[c]) * ndof + db] += rows[t];
-                }
-            } else if (lane == 0) {
-                for (int t = 0; t < ndof * N; ++t) {
-                    int da = t / N, col = t - da * N;
-                    int c = col / ndof, db = col - c * ndof;
-                    acc[da * rowlen + int(map[c]) * ndof + db] += rows[t];
+            const unsigned key = gl < nn ? (unsigned(grp) << 16 | map[gl]) : 0x80000000u | lane;
+            const unsigned same = __match_any_sync(0xffffffffu, key);
+            const unsigned twice = __ballot_sync(0xffffffffu, (same & (same - 1)) != 0);
+            const unsigned mine = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (grp * G);
+            if (!(twice & mine)) {
+                if (nn == 8) add_rows<ND, 8, G>(acc, rowlen, map, rows, gl);
+                else if (nn == 4) add_rows<ND, 4, G>(acc, rowlen, map, rows, gl);
+                else if (nn == 3) add_rows<ND, 3, G>(acc, rowlen, map, rows, gl);
+                else
+                    for (int t = gl; t < ND * N; t += G) {
+                        const int da = t / N, col = t - da * N, c = col / ND, db = col - c * ND;
+                        acc[da * rowlen + int(map[c]) * ND + db] += rows[t];
+                    }
+            } else if (gl == 0) {
+                for (int t = 0; t < ND * N; ++t) {
+                    const int da = t / N, col = t - da * N, c = col / ND, db = col - c * ND;
+                    acc[da * rowlen + int(map[c]) * ND + db] += rows[t];
                 }
             }
             __syncwarp();
         }
-        for (int q = lane; q < total; q += 32) vals[base + q] = acc[q];
+        for (int q = gl; q < total; q += G) vals[base + q] = acc[q];
         __syncwarp();
     }
 }
@@ -216,20 +247,25 @@ void assemble_values(svx_ctx* ctx, svx_op* op, const double* ke, int ke_stride, 
     const Pattern& P = op->pat;
     if (op->n_nodes == 0) return;
     const int acc_stride = op->ndof * op->ndof * std::max(1, P.max_deg);
-    int warps = ASM_WARPS;
-    size_t smem = size_t(warps) * acc_stride * sizeof(double);
-    if (smem > 200 * 1024)
+    const int per = op->ndof == 1 ? 4 : 1;  // nodes a warp
+    if (size_t(ASM_WARPS) * acc_stride * sizeof(double) > 200 * 1024)
         throw ModelFail{SVX_INVALID_MODEL, 0, -1,
                         "node degree " + std::to_string(P.max_deg) +
                             " exceeds the shared-memory block of the assembly kernel"};
+    int warps = ASM_WARPS;  // fewer where four nodes a warp of a large degree need the room
+    while (warps > 1 && size_t(warps) * per * acc_stride * sizeof(double) > 200 * 1024) warps /= 2;
+    const size_t smem = size_t(warps) * per * acc_stride * sizeof(double);
+    auto* const kernel = op->ndof == 3   ? &assemble_kernel<3>
+                         : op->ndof == 2 ? &assemble_kernel<2>
+                                         : &assemble_kernel<1>;
     if (smem > 48 * 1024)
-        SVX_CUDA(cudaFuncSetAttribute(assemble_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      int(smem)));
-    int64_t blocks = (op->n_nodes + warps - 1) / warps;
+        SVX_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel),
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    int64_t blocks = (op->n_nodes + warps * per - 1) / (warps * per);
     int64_t cap = int64_t(ctx->sm_count) * 32;
     if (blocks > cap) blocks = cap;
-    assemble_kernel<<<unsigned(blocks), warps * 32, smem, ctx->stream>>>(
-        op->n_nodes, op->ndof, P.max_nn, acc_stride, P.slot_ptr.p, P.slot_elem.p, P.slot_local.p,
+    kernel<<<unsigned(blocks), warps * 32, smem, ctx->stream>>>(
+        op->n_nodes, P.max_nn, acc_stride, P.slot_ptr.p, P.slot_elem.p, P.slot_local.p,
         P.slot_map.p, op->conn_ptr.p, P.adj_ptr.p, P.node_base.p, ke, ke_stride, vals);
     SVX_LAUNCH_CHECK();
 }
