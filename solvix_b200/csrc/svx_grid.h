@@ -6,6 +6,7 @@
 #ifdef __CUDACC__
 
 #include "svx_internal.h"
+#include "svx_warp.h"
 
 namespace svx {
 
@@ -61,6 +62,47 @@ __device__ __forceinline__ bool grid_sync(GridBarrier* gb, unsigned int nblocks,
     }
     __syncthreads();
     return ok != 0;
+}
+
+// Sums of (a, b) over the grid, the same bits in every thread: warp sums on
+// the tensor cores, the block's pair to `pt` (one pair a block, 16-byte
+// aligned), the barrier, and one warp reads the other blocks' pairs (read by
+// all warps of 148 blocks their few cache lines are a hot spot of the L2).
+// sh: 66 doubles.  The reductions of an iteration use different `pt`: a block
+// past the first one's barrier may publish its next pair while a late block
+// still reads this one; with a barrier between two uses of a `pt` no block can
+// overwrite what another still reads.
+__device__ __forceinline__ bool grid_pair_sum(GridBarrier* gb, unsigned int nblocks,
+                                              unsigned int& target, double* pt, double* sh,
+                                              double a, double b, double& ta, double& tb) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = int(blockDim.x) >> 5;
+    const double v = lane_sum_pair(a, b, lane);
+    if ((lane & 15) == 0) sh[2 * warp + (lane >> 4)] = v;
+    __syncthreads();
+    if (warp == 0) {
+        const double w = lane_sum_pair(lane < warps ? sh[2 * lane] : 0.0,
+                                       lane < warps ? sh[2 * lane + 1] : 0.0, lane);
+        if ((lane & 15) == 0) pt[2 * blockIdx.x + (lane >> 4)] = w;
+    }
+    if (!grid_sync(gb, nblocks, target)) return false;
+    if (warp == 0) {
+        double x = 0.0, y = 0.0;
+        for (int k = lane; k < int(nblocks); k += 32) {
+            const double2 w = __ldcg(reinterpret_cast<const double2*>(pt) + k);
+            x += w.x;
+            y += w.y;
+        }
+        x = lane_sum(x);
+        y = lane_sum(y);
+        if (lane == 0) {
+            sh[64] = x;
+            sh[65] = y;
+        }
+    }
+    __syncthreads();
+    ta = sh[64];
+    tb = sh[65];
+    return true;
 }
 
 }  // namespace svx

@@ -33,7 +33,6 @@
 
 #include "svx_internal.h"
 #include "svx_grid.h"
-#include "svx_warp.h"
 
 #include <cooperative_groups.h>
 
@@ -1387,7 +1386,7 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
                 double* part, PcgScalars* s, GridBarrier* gb, int chunk, int nodes_cap,
                 int max_deg, int stage, int first) {
     extern __shared__ __align__(16) unsigned char svx_dyn_smem[];
-    __shared__ double sh[64];
+    __shared__ double sh[66];
     // block-uniform values kept out of registers: ||f||, tol, the last
     // iterate's ||r|| / ||f|| and r.r (thread 0 keeps them), the reliable
     // update's r.r, max_iter
@@ -1470,45 +1469,12 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
     const int gl = lane & (G - 1), grp = lane / G;
     const bool writer = (blockIdx.x == 0 && threadIdx.x == 0);
     __syncthreads();
-    // sum over the grid of the block partials (a, b), published in slot
-    // `slot` of `part`.  The two reductions of an iteration use two slots: a
-    // block past the first one's barrier may publish its second partials
-    // while a late block still reads the first ones; with a barrier between
-    // two uses of a slot no block can overwrite what another still reads.
-    // Warp sums on the tensor cores, and one warp reads the other blocks'
-    // partials: read by all 16 warps of 148 blocks their few cache lines are
-    // a hot spot of the L2.  (Posting the sums as numbered words that every
-    // block polls, instead of the counting barrier, measured slower: 8.8
-    // against 7.2 us an iteration at 81 nodes, 12.4 against 8.2 at 6,561.)
+    // the two reductions of an iteration use two slots of `part`.  (Posting the
+    // sums as numbered words that every block polls, instead of the counting
+    // barrier, measured slower: 8.8 against 7.2 us an iteration at 81 nodes,
+    // 12.4 against 8.2 at 6,561.)
     auto grid_totals = [&](int slot, double a, double b, double& ta, double& tb) -> bool {
-        double* pt = part + size_t(slot) * 2 * B;
-        const double v = lane_sum_pair(a, b, lane);
-        if ((lane & 15) == 0) sh[2 * warp + (lane >> 4)] = v;
-        __syncthreads();
-        if (warp == 0) {
-            const double w = lane_sum_pair(lane < W ? sh[2 * lane] : 0.0,
-                                           lane < W ? sh[2 * lane + 1] : 0.0, lane);
-            if ((lane & 15) == 0) pt[2 * blockIdx.x + (lane >> 4)] = w;
-        }
-        if (!grid_sync(gb, B, bar_target)) return false;
-        if (warp == 0) {
-            double x = 0.0, y = 0.0;
-            for (int k = lane; k < int(B); k += 32) {
-                const double2 w = __ldcg(reinterpret_cast<const double2*>(pt) + k);
-                x += w.x;
-                y += w.y;
-            }
-            x = lane_sum(x);
-            y = lane_sum(y);
-            if (lane == 0) {
-                sh[32] = x;
-                sh[33] = y;
-            }
-        }
-        __syncthreads();
-        ta = sh[32];
-        tb = sh[33];
-        return true;
+        return grid_pair_sum(gb, B, bar_target, part + size_t(slot) * 2 * B, sh, a, b, ta, tb);
     };
     if (ALG == 1 && first) {
         // neighbours gather z and the previous p (zero): store z, barrier
@@ -1647,6 +1613,172 @@ pcg_smem_kernel(int64_t n_nodes, const int64_t* __restrict__ adj_ptr,
     finish(PCG_RUNNING);
 }
 
+
+// ------------------------------------------------------------ one dof a node
+// The persistent PCG of conduction systems.  A scalar row has one value a
+// neighbour, so with several lanes a node (pcg_smem_kernel) the loads of the
+// gathers bound it: eight lanes a node, four nodes a warp touch a dozen cache
+// lines a load, 22.5 us an iteration at 240 x 24 x 24.  Here a lane owns a
+// node and a warp a slice of 32 consecutive nodes, K stored slice by slice
+// with the neighbour slot outermost ([slice][slot][lane], rows padded with
+// zeros to the largest degree), so a warp reads K and its columns in full
+// lines and, the k-th neighbours of consecutive nodes being consecutive nodes
+// in a structured mesh, gathers nearly so, through the L1 (the grid barrier's
+// acquire leaves no stale line there).  z and the previous p are one pair, so
+// that a neighbour is one load: the pairs of an iteration are written before
+// its second barrier and gathered only before the next one's first, so one
+// buffer is enough.  Two barriers an iteration as in ALG 1 above, whose
+// recurrence this is: 10.7 us an iteration at 240 x 24 x 24 (3.48 ms a solve
+// of 326, 7.35 before), of which the two grid sums take 5 and reading K
+// (33 MB) from the L2 most of the rest; 7.0 at 120 x 12 x 12 (8.8 before).
+// 1,024 threads a block, 5 or 14 neighbours in flight, and the columns left
+// in the L2 measured within 5% of this or slower.
+constexpr int SCALAR_THREADS = 512;
+constexpr int SCALAR_BATCH = 9;  // neighbours in flight: a third of a solid's 27, a plate's 9
+constexpr size_t SCALAR_SMEM = 200 * 1024;
+// Rows wider than a solid's 27 keep pcg_smem_kernel, and so does a system that
+// padding every row to the widest would make more than twice as large (the
+// kernel streams it each iteration; a small one is not bound by that).
+constexpr int SCALAR_MAX_DEG = 32;
+constexpr int64_t SCALAR_SMALL = 65536;
+
+__global__ void slice_rows_kernel(int64_t n, int width, const int64_t* __restrict__ adj_ptr,
+                                  const int32_t* __restrict__ adj,
+                                  const int64_t* __restrict__ node_base,
+                                  const double* __restrict__ vals, double* __restrict__ out,
+                                  int32_t* __restrict__ cols) {
+    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;  // rounded up to slices
+    const int64_t s = i / 32, lane = i % 32;
+    if (s * 32 >= n) return;
+    const int64_t a0 = i < n ? adj_ptr[i] : 0;
+    const int d = i < n ? int(adj_ptr[i + 1] - a0) : 0;
+    const int32_t self = int32_t(i < n ? i : n - 1);
+    const double* v = i < n ? vals + node_base[i] : vals;
+    for (int k = 0; k < width; ++k) {
+        const int64_t at = (s * width + k) * 32 + lane;
+        // a node no element uses has a row of its diagonal alone
+        out[at] = k < d ? v[k] : (d == 0 && i < n && k == 0 ? v[0] : 0.0);
+        cols[at] = k < d ? adj[a0 + k] : self;
+    }
+}
+
+template <int PB>
+__global__ void __launch_bounds__(PB, 1)
+pcg_scalar_kernel(int64_t n, int width, const double* __restrict__ vals,
+                  const int32_t* __restrict__ cols, const double* __restrict__ inv_diag,
+                  double* u_g, double* r_g, double2* zp, double* part, PcgScalars* s,
+                  GridBarrier* gb, int chunk, int cap, int cols_here, int first) {
+    extern __shared__ __align__(16) unsigned char svx_dyn_smem[];
+    __shared__ double sh[66];
+    constexpr int W = PB / 32, U = SCALAR_BATCH;
+    const unsigned int B = gridDim.x;
+    unsigned int bar_target = 0;
+    volatile PcgScalars* vs = s;
+    if (vs->status != PCG_RUNNING) return;
+    const int slices = int((n + 31) / 32);
+    const int s0 = int(int64_t(slices) * blockIdx.x / B),
+              s1 = int(int64_t(slices) * (blockIdx.x + 1) / B);
+    const int row0 = s0 * 32, rows = min(int(n), s1 * 32) - row0;
+    double* u_s = reinterpret_cast<double*>(svx_dyn_smem);
+    double* r_s = u_s + cap;
+    double* p_s = r_s + cap;
+    double* q_s = p_s + cap;
+    double* z_s = q_s + cap;
+    double* d_s = z_s + cap;
+    int32_t* c_s = reinterpret_cast<int32_t*>(d_s + cap);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const double bnorm = vs->bnorm, tol = vs->tol;
+    const long long max_iter = vs->max_iter;
+    long long it = vs->it;
+    double rz = vs->rz, beta = vs->beta, rr = vs->rr, res = vs->res;
+    if (first) beta = 0.0;
+    for (int t = threadIdx.x; t < rows; t += PB) {
+        const int row = row0 + t;
+        const double di = inv_diag[row], ri = r_g[row];
+        d_s[t] = di;
+        r_s[t] = ri;
+        z_s[t] = ri * di;
+        u_s[t] = u_g[row];
+        p_s[t] = first ? 0.0 : zp[row].y;
+        if (first) zp[row] = make_double2(ri * di, 0.0);
+    }
+    if (cols_here)
+        for (int t = threadIdx.x; t < (s1 - s0) * width * 32; t += PB)
+            c_s[t] = cols[int64_t(s0) * width * 32 + t];
+    if (!grid_sync(gb, B, bar_target)) return;
+    int status = PCG_RUNNING;
+    for (int c = 0; c < chunk && status == PCG_RUNNING; ++c) {
+        for (int sl = s0 + warp; sl < s1; sl += W) {
+            const double* v = vals + int64_t(sl) * width * 32 + lane;
+            const int32_t* cl = cols_here ? c_s + (sl - s0) * width * 32 + lane
+                                          : cols + int64_t(sl) * width * 32 + lane;
+            double acc[3] = {0.0, 0.0, 0.0};
+            int k = 0;
+            for (; k + U <= width; k += U) {
+                double kv[U];
+                double2 x[U];
+#pragma unroll
+                for (int m = 0; m < U; ++m) kv[m] = __ldg(v + (k + m) * 32);
+#pragma unroll
+                for (int m = 0; m < U; ++m) x[m] = zp[cl[(k + m) * 32]];
+#pragma unroll
+                for (int m = 0; m < U; ++m) acc[m % 3] += kv[m] * __fma_rn(beta, x[m].y, x[m].x);
+            }
+            for (; k < width; ++k) {
+                const double2 x = zp[cl[k * 32]];
+                acc[0] += __ldg(v + k * 32) * __fma_rn(beta, x.y, x.x);
+            }
+            const int t = (sl - s0) * 32 + lane;
+            if (t < rows) q_s[t] = (acc[0] + acc[1]) + acc[2];
+        }
+        __syncthreads();
+        double pq = 0.0, pap, unused;
+        for (int t = threadIdx.x; t < rows; t += PB) {
+            const double pi = __fma_rn(beta, p_s[t], z_s[t]);
+            p_s[t] = pi;
+            pq += pi * q_s[t];
+        }
+        if (!grid_pair_sum(gb, B, bar_target, part, sh, pq, 0.0, pap, unused)) return;
+        if (!(pap > 0.0)) {  // p.Kp <= 0 or NaN: breakdown
+            it += 1;
+            status = PCG_BREAKDOWN;
+            break;
+        }
+        const double alpha = rz / pap;
+        double lrr = 0.0, lrz = 0.0, rz_new;
+        for (int t = threadIdx.x; t < rows; t += PB) {
+            const double pi = p_s[t];
+            u_s[t] += alpha * pi;
+            const double ri = r_s[t] - alpha * q_s[t];
+            const double zi = ri * d_s[t];
+            r_s[t] = ri;
+            z_s[t] = zi;
+            zp[row0 + t] = make_double2(zi, pi);
+            lrr += ri * ri;
+            lrz += ri * zi;
+        }
+        if (!grid_pair_sum(gb, B, bar_target, part + 2 * size_t(B), sh, lrr, lrz, rr, rz_new))
+            return;
+        it += 1;
+        res = sqrt(rr) / bnorm;
+        beta = rz_new / rz;
+        rz = rz_new;
+        status = res <= tol ? PCG_CONVERGED : it >= max_iter ? PCG_MAXITER : PCG_RUNNING;
+    }
+    for (int t = threadIdx.x; t < rows; t += PB) {
+        u_g[row0 + t] = u_s[t];
+        r_g[row0 + t] = r_s[t];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        s->it = it;
+        s->res = res;
+        s->rr = rr;
+        s->rz = rz;
+        s->beta = beta;
+        __threadfence();
+        if (status != PCG_RUNNING) s->status = status;
+    }
+}
 
 // ------------------------------------------------------------ batched PCG
 // Thousands of independent models concatenated into one block-diagonal
@@ -2656,6 +2788,86 @@ struct PcgRun {
         }
     }
 
+    // The persistent form of one dof a node (pcg_scalar_kernel).  Returns -1
+    // without launching when the rows do not fit its slices, a block's vectors
+    // its shared memory or the slices the device.
+    int iterate_scalar(int chunk) {
+        if constexpr (std::is_same<M, double>::value && std::is_same<V, double>::value &&
+                      std::is_same<U, double>::value) {
+            cudaStream_t st = ctx->stream;
+            constexpr int PB = SCALAR_THREADS;
+            const int width = std::max(op->pat.max_deg, 1);
+            int coop = 0;
+            SVX_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device));
+            if (!coop || op->ndof != 1 || width > SCALAR_MAX_DEG) return -1;
+            const int64_t slices = (n + 31) / 32, padded = slices * width * 32;
+            if (padded > std::max(2 * op->pat.nnz, SCALAR_SMALL)) return -1;
+            const unsigned int B = unsigned(std::min<int64_t>(ctx->sm_count, slices));
+            int cap = int((slices + B - 1) / B) * 32;
+            size_t smem = size_t(cap) * 6 * sizeof(double);
+            if (smem > SCALAR_SMEM) return -1;
+            // the columns stay in shared memory where they fit
+            int cols_here = smem + size_t(cap) * width * sizeof(int32_t) <= SCALAR_SMEM;
+            if (cols_here) smem += size_t(cap) * width * sizeof(int32_t);
+            void* fn = (void*)pcg_scalar_kernel<PB>;
+            SVX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          int(SCALAR_SMEM)));
+            DBuf<double> part, sv;
+            DBuf<double2> zp;
+            DBuf<int32_t> sc;
+            DBuf<GridBarrier> gb;
+            part.alloc(ctx->pool, 4 * size_t(B) + 2);
+            gb.alloc(ctx->pool, 1);
+            try {
+                zp.alloc(ctx->pool, n);
+                sv.alloc(ctx->pool, padded);
+                sc.alloc(ctx->pool, padded);
+            } catch (const ModelFail& f) {  // a full device: the rows stay where they are
+                if (f.code != SVX_OOM) throw;
+                return -1;
+            }
+            SVX_CUDA(cudaMemsetAsync(gb.p, 0, sizeof(GridBarrier), st));
+            // rows past n repeat the last node with a zero: any finite pair will do there
+            slice_rows_kernel<<<unsigned((slices * 32 + BLOCK - 1) / BLOCK), BLOCK, 0, st>>>(
+                n, width, op->pat.adj_ptr.p, op->pat.adj.p, op->pat.node_base.p, vals, sv.p, sc.p);
+            SVX_LAUNCH_CHECK();
+            int64_t rows = n;
+            int w = width, first = 1;
+            GridBarrier* gbp = gb.p;
+            void* args[] = {&rows, &w, &sv.p, &sc.p, (void*)&inv_diag, (void*)&u, (void*)&r,
+                            &zp.p, &part.p, (void*)&s, (void*)&gbp, (void*)&chunk, &cap,
+                            &cols_here, &first};
+            SVX_CUDA(cudaMemcpyAsync(h_s, s, sizeof(PcgScalars), cudaMemcpyDeviceToHost, st));
+            SVX_CUDA(cudaStreamSynchronize(st));
+            const long long launches_max = h_s->max_iter / chunk + 2;
+            GridBarrier hgb{};
+            int status = h_s->status;
+            for (long long launch = 0; status == PCG_RUNNING; ++launch) {
+                if (launch >= launches_max)
+                    throw ModelFail{SVX_CUDA_ERROR, 0, -1,
+                                    "PCG status did not leave RUNNING within max_iter"};
+                SVX_CUDA(cudaMemsetAsync(&gbp->count, 0, sizeof(unsigned int), st));
+                SVX_CUDA(cudaLaunchCooperativeKernel(fn, dim3(B), dim3(PB), args, smem, st));
+                g_launches.fetch_add(1, std::memory_order_relaxed);
+                first = 0;
+                SVX_CUDA(cudaMemcpyAsync(h_s, s, sizeof(PcgScalars), cudaMemcpyDeviceToHost,
+                                         st));
+                SVX_CUDA(cudaMemcpyAsync(&hgb, gbp, sizeof(GridBarrier), cudaMemcpyDeviceToHost,
+                                         st));
+                SVX_CUDA(cudaStreamSynchronize(st));
+                if (hgb.error)
+                    throw ModelFail{SVX_CUDA_ERROR, 0, -1,
+                                    "persistent PCG: a grid barrier wait ran out (blocks not "
+                                    "co-resident)"};
+                status = h_s->status;
+            }
+            return status;
+        } else {
+            (void)chunk;
+            return -1;
+        }
+    }
+
     // The persistent form on bricks of elements (svx_brick.cu): cooperative
     // launches of up to `chunk` iterations each.
     int iterate_brick(int chunk) {
@@ -3095,7 +3307,8 @@ PcgResult pcg_fp64(svx_ctx* ctx, svx_op* op, double tol, long long max_iter, int
         // the graph form starts from the init kernel's p = z0 too: a
         // persistent launch that cannot start leaves p untouched
         status = -1;
-        if (!graph && ctx->pcg_smem)
+        if (!graph && ctx->pcg_smem) status = run.iterate_scalar(persistent_chunk(op->pat.nnz));
+        if (!graph && status < 0 && ctx->pcg_smem)
             status = run.iterate_smem(persistent_chunk(op->pat.nnz), transposed_values(ctx, op));
         if (!graph && status < 0) status = run.iterate_persistent(persistent_chunk(op->pat.nnz));
         if (status < 0) status = run.iterate(check_every);
