@@ -9,8 +9,8 @@
 // one block column per step:
 //
 //   panel kernel   every block factors the diagonal tile (J, J) into L_JJ and
-//                  D_J (the whole block, in shared memory, one column per
-//                  step); block 0 stores them apart from the band (the
+//                  D_J (the whole block, entries in registers, one column
+//                  per step); block 0 stores them apart from the band (the
 //                  other blocks are still reading tile (J, J)); block g
 //                  solves the panel tile (J+1+g, J): W = A L_JJ^-T,
 //                  L = W D_J^-1;
@@ -23,7 +23,8 @@
 // D_i <= 1e-13 * max(max_j |K_ij|, DBL_MIN) fails with the reference's
 // message and equation number (i in the RCM order); the first failing
 // equation is kept with an atomic minimum.  The forward, diagonal and
-// backward solves run in one block, block row by block row.
+// backward solves run in one block up to 16 tiles of bandwidth, over the
+// whole GPU beyond, block row by block row.
 //
 // The summation order differs from the reference's up-looking one, so D, u
 // and the residual agree with it to rounding (D to a few ulps times the
@@ -122,61 +123,74 @@ ldlt_panel_kernel(int64_t J, int64_t n, int w, int wj, double* __restrict__ band
                   double* __restrict__ dvec, const double* __restrict__ row_max,
                   unsigned long long* fail) {
     __shared__ double s_l[LT][LT + 1];
+    __shared__ double s_col[2][LT];
+    __shared__ double s_lim[LT];
     __shared__ int s_flag;
-    if (stopped(fail, &s_flag)) return;
-    const double* dt = band + tile_off(J, 0, w);
-    for (int k = threadIdx.x; k < LT2; k += LBLOCK) s_l[k / LT][k % LT] = dt[k];
-    __syncthreads();
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    // Right-looking LDL^T of the tile in shared memory, the whole block at
-    // once: at column c every entry (r, k), c < k <= r, takes
-    // A[r][k] -= (W[r][c] / D_c) W[k][c] with W column c still unscaled,
-    // then column c becomes L = W / D_c; so each entry gets
-    // A[r][k] - sum_c L[r][c] W[k][c] in column order.
+    const int r = threadIdx.x >> 3, g = threadIdx.x & 7;
+    const int d = 1 + int(blockIdx.x);
+    const double* dt = band + tile_off(J, 0, w);
+    double* tile = band + tile_off(J + d, d, w);
+    double a[4], x[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) a[j] = dt[r * LT + g + 8 * j];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x[q] = d <= wj ? tile[(warp + 8 * q) * LT + lane] : 0.0;
+    if (threadIdx.x < LT) s_lim[threadIdx.x] = 1e-13 * fmax(row_max[J * LT + threadIdx.x], DBL_MIN);
+    if (stopped(fail, &s_flag)) return;
+    // Right-looking LDL^T of the tile, the whole block at once, thread (r, g)
+    // with the entries (r, g + 8 j) in registers: at column c every entry
+    // (r, k), c < k <= r, takes A[r][k] -= (W[r][c] / D_c) W[k][c] with W
+    // column c still unscaled, then column c becomes L = W / D_c; so each
+    // entry gets A[r][k] - sum_c L[r][c] W[k][c] in column order.  The columns
+    // pass through shared memory, the next one written by its owners as soon
+    // as it is final: one barrier and one division a column (the chain that
+    // bounds this kernel at a small bandwidth; at 7 tiles 11.3 us a step under
+    // the profiler, 19.3 with two of each and the pivots' limits read from
+    // global memory in the chain; rolled, 15.0).
+    if (g == 0) s_col[0][r] = a[0];
+    __syncthreads();
+#pragma unroll
     for (int c = 0; c < LT; ++c) {
-        const double dc = s_l[c][c];
+        const double* col = s_col[c & 1];
+        const double dc = col[c];
         const int64_t eq = J * LT + c;
         if (threadIdx.x == 0 && blockIdx.x == 0 && eq < n) {
-            const double lim = 1e-13 * fmax(row_max[eq], DBL_MIN);
-            if (!isfinite(dc) || dc <= lim)
+            if (!isfinite(dc) || dc <= s_lim[c])
                 atomicMin(fail, (unsigned long long)(eq) << 1 | (dc < 0.0 ? 1ull : 0ull));
         }
-        {
-            // thread (r, g) takes row r, columns c + 1 + g, c + 9 + g, ... <= r
-            const int r = threadIdx.x >> 3, g = threadIdx.x & 7;
-            if (r > c) {
-                const double l = s_l[r][c] / dc;
-                for (int k = c + 1 + g; k <= r; k += 8) s_l[r][k] -= l * s_l[k][c];
-            }
+        const double l = col[r] / dc;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int k = g + 8 * j;
+            if (k > c && k <= r) a[j] -= l * col[k];
+            if (k == c && r > c) a[j] = l;
+            if (k == c + 1) s_col[(c + 1) & 1][r] = a[j];
         }
-        __syncthreads();
-        if (threadIdx.x > c && threadIdx.x < LT) s_l[threadIdx.x][c] /= dc;
         __syncthreads();
     }
     if (blockIdx.x == 0) {
         double* out = dfac + size_t(J) * LT2;
-        for (int k = threadIdx.x; k < LT2; k += LBLOCK) out[k] = s_l[k / LT][k % LT];
-        if (threadIdx.x < LT) dvec[J * LT + threadIdx.x] = s_l[threadIdx.x][threadIdx.x];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            out[r * LT + g + 8 * j] = a[j];
+            if (g + 8 * j == r) dvec[J * LT + r] = a[j];
+        }
     }
-    const int d = 1 + int(blockIdx.x);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) s_l[r][g + 8 * j] = a[j];
+    __syncthreads();
     if (d > wj) return;
     // Panel tile (J + d, J): warp w takes rows w, w + 8, w + 16, w + 24
-    // together; lane c' keeps row c' of L_JJ in registers and ends with
+    // together; lane c' takes row c' of L_JJ and ends with
     // W[row][c'] = A[row][c'] - sum_{c < c'} W[row][c] L_JJ[c'][c].
     static_assert(LT == 4 * (LBLOCK / 32), "four panel rows per warp");
-    double lrow[LT];
-#pragma unroll
-    for (int k = 0; k < LT; ++k) lrow[k] = s_l[lane][k];
     const double dl = s_l[lane][lane];
-    double* tile = band + tile_off(J + d, d, w);
     double* wt = panel + size_t(d - 1) * LT2;
-    double x[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) x[q] = tile[(warp + 8 * q) * LT + lane];
-#pragma unroll
+#pragma unroll 4
     for (int c = 0; c < LT; ++c) {
-        const double lc = lrow[c];
+        const double lc = s_l[lane][c];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const double v = __shfl_sync(0xffffffffu, x[q], c);
@@ -348,6 +362,165 @@ ldlt_solve_kernel(int64_t n, int64_t nb, int w, const double* __restrict__ band,
         __syncthreads();
     }
     for (int64_t r = threadIdx.x; r < n; r += SBLOCK) u[r] = y[perm[r]];
+}
+
+// The same in one block for bandwidths of up to 16 tiles, one barrier a block
+// row: a grid barrier a block row was most of the cooperative form below
+// there (828 us of the 40 x 4 x 4 cantilever's solve at 7 tiles, 413 here).
+// Beyond, a second tile a warp no longer hides under the chain: a first form
+// with them took 25% longer than the cooperative one at 22 tiles.  Warp
+// 0 walks the chain: row I's sum, less T(I, 1) y_(I-1), then the diagonal tile
+// by shuffles, both tiles in shared memory since the row before.  Meanwhile
+// warp p >= 1 takes tile 1 + p of row I + 1, whose y are final, and all warps
+// but 0 copy its two tiles of the chain.
+constexpr int NBLOCK = 512;
+constexpr int NWARPS = NBLOCK / 32;
+constexpr int NARROW_BLOCKS = NWARPS;  // tiles 2 .. NWARPS, one a warp
+constexpr int RING = 32;
+static_assert(RING > NARROW_BLOCKS + 1 && (RING & (RING - 1)) == 0, "the rows still needed");
+constexpr size_t NARROW_SMEM =
+    sizeof(double) * (4 * LT * (LT + 1) + (2 * NWARPS + RING) * LT);
+__device__ __forceinline__ void copy8(double* to, const double* from) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                     unsigned(__cvta_generic_to_shared(to))), "l"(from) : "memory");
+}
+__global__ void __launch_bounds__(NBLOCK)
+ldlt_solve_narrow_kernel(int64_t n, int64_t nb, int w, const double* __restrict__ band,
+                         const double* __restrict__ dfac, const double* __restrict__ dvec,
+                         const int32_t* __restrict__ perm, const double* __restrict__ f,
+                         double* y, double* __restrict__ u, const unsigned long long* fail) {
+    extern __shared__ __align__(16) double s_dyn[];
+    double* s_diag = s_dyn;                          // [2][LT][LT + 1]
+    double* s_next = s_diag + 2 * LT * (LT + 1);     // [2][LT][LT + 1]
+    double* s_part = s_next + 2 * LT * (LT + 1);     // [2][NWARPS][LT]
+    double* s_y = s_part + 2 * NWARPS * LT;          // [RING][LT]: the last rows solved
+    __shared__ int s_flag;
+    if (stopped(fail, &s_flag)) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t rows = nb * LT;
+    for (int64_t i = threadIdx.x; i < rows; i += NBLOCK) y[i] = 0.0;
+    __syncthreads();
+    for (int64_t r = threadIdx.x; r < n; r += NBLOCK) y[perm[r]] = f[r];
+    // the chain's tiles of row R to their half of the buffers: the diagonal's
+    // and, for another row before it (off: its off-diagonal tile), that one
+    auto fetch = [&](int64_t R, const double* off) {
+        double* to = s_diag + (R & 1) * LT * (LT + 1);
+        const double* from = dfac + size_t(R) * LT2;
+        if (warp == 0) return;
+        for (int k = threadIdx.x - 32; k < LT2; k += NBLOCK - 32)
+            copy8(to + (k / LT) * (LT + 1) + k % LT, from + k);
+        to = s_next + (R & 1) * LT * (LT + 1);
+        if (off)
+            for (int k = threadIdx.x - 32; k < LT2; k += NBLOCK - 32)
+                copy8(to + (k / LT) * (LT + 1) + k % LT, off + k);
+    };
+    auto fetched = [&]() {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+    };
+    // row R's tile d >= 2 of warp d - 1, on the FP64 tensor cores, in 8 x 4
+    // pieces (whole sectors a load; a lane a row reads 32 of them) times x in
+    // the first column of B.  The tile is read an iteration ahead.
+    const int fr = lane >> 2, fc = lane & 3, d = 1 + warp;
+    double tv[LT / 4][4];
+    auto read_tile = [&](int64_t R, int dmax, bool trans) {
+        if (warp == 0 || d > dmax) return;
+        const double* t = band + (trans ? tile_off(R + d, d, w) + fc * LT + fr
+                                        : tile_off(R, d, w) + fr * LT + fc);
+        const int sk = trans ? 4 * LT : 4, sr = trans ? 8 : 8 * LT;
+#pragma unroll
+        for (int k = 0; k < LT / 4; ++k)
+#pragma unroll
+            for (int rb = 0; rb < 4; ++rb) tv[k][rb] = __ldg(t + k * sk + rb * sr);
+    };
+    auto partial = [&](int64_t R, int dmax, bool trans) {
+        double q[4][2] = {};
+        if (d <= dmax) {
+            const double* xv = s_y + ((trans ? R + d : R - d) & (RING - 1)) * LT + fc;
+#pragma unroll
+            for (int k = 0; k < LT / 4; ++k) {
+                const double xk = fr == 0 ? xv[4 * k] : 0.0;
+#pragma unroll
+                for (int rb = 0; rb < 4; ++rb) dmma(q[rb][0], q[rb][1], tv[k][rb], xk);
+            }
+        }
+        if (fc == 0)
+#pragma unroll
+            for (int rb = 0; rb < 4; ++rb)
+                s_part[((R & 1) * NWARPS + warp) * LT + 8 * rb + fr] = q[rb][0];
+    };
+    // row R's sum of all tiles d >= 1 (warp 0); last: the row before it
+    auto row_sum = [&](int64_t R, double last, bool has, bool trans) -> double {
+        double tot = 0.0;
+        if (has) {
+            const double* t = s_next + (R & 1) * LT * (LT + 1);
+            double q[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int k = 0; k < LT; ++k)
+                q[k & 3] += (trans ? t[k * (LT + 1) + lane] : t[lane * (LT + 1) + k]) *
+                            __shfl_sync(0xffffffffu, last, k);
+            tot = (q[0] + q[1]) + (q[2] + q[3]);
+        }
+        double more = 0.0;
+        for (int p = 1; p < NWARPS && p < w; ++p) more += s_part[((R & 1) * NWARPS + p) * LT + lane];
+        return tot + more;
+    };
+    auto above = [&](int64_t R) { return int(R < w ? R : w); };  // tiles of row R
+    auto below = [&](int64_t R) { return int(nb - 1 - R < w ? nb - 1 - R : w); };
+    double x = 0.0;
+    fetch(0, nullptr);
+    if (warp) partial(0, 0, false);
+    fetched();
+    double rhs = __ldcg(y + lane);  // of the row to come
+    for (int64_t I = 0; I < nb; ++I) {
+        if (I + 1 < nb) fetch(I + 1, w >= 1 ? band + tile_off(I + 1, 1, w) : nullptr);
+        if (warp == 0) {
+            const double yi = rhs;
+            if (I + 1 < nb) rhs = __ldcg(y + (I + 1) * LT + lane);
+            x = yi - row_sum(I, x, I >= 1 && w >= 1, false);
+            const double* t = s_diag + (I & 1) * LT * (LT + 1) + lane * (LT + 1);
+#pragma unroll
+            for (int c = 0; c < LT; ++c) {
+                const double v = __shfl_sync(0xffffffffu, x, c);
+                if (lane > c) x -= t[c] * v;
+            }
+            y[I * LT + lane] = x;
+            s_y[(I & (RING - 1)) * LT + lane] = x;
+        } else {
+            if (I + 1 < nb) partial(I + 1, above(I + 1), false);
+            if (I + 2 < nb) read_tile(I + 2, above(I + 2), false);
+        }
+        fetched();
+    }
+    fetch(nb - 1, nullptr);
+    if (warp) partial(nb - 1, 0, true);
+    rhs = x;
+    double piv = dvec[(nb - 1) * LT + lane];
+    fetched();
+    for (int64_t J = nb - 1; J >= 0; --J) {
+        if (J >= 1) fetch(J - 1, w >= 1 ? band + tile_off(J, 1, w) : nullptr);
+        if (warp == 0) {
+            const double yj = rhs / piv;
+            if (J >= 1) {
+                rhs = __ldcg(y + (J - 1) * LT + lane);
+                piv = dvec[(J - 1) * LT + lane];
+            }
+            x = yj - row_sum(J, x, J + 1 < nb && w >= 1, true);
+            const double* t = s_diag + (J & 1) * LT * (LT + 1) + lane;
+#pragma unroll
+            for (int r = LT - 1; r >= 0; --r) {
+                const double v = __shfl_sync(0xffffffffu, x, r);
+                if (lane < r) x -= t[r * (LT + 1)] * v;
+            }
+            y[J * LT + lane] = x;
+            s_y[(J & (RING - 1)) * LT + lane] = x;
+        } else {
+            if (J >= 1) partial(J - 1, below(J - 1), true);
+            if (J >= 2) read_tile(J - 2, below(J - 2), true);
+        }
+        fetched();
+    }
+    for (int64_t r = threadIdx.x; r < n; r += NBLOCK) u[r] = __ldcg(y + perm[r]);
 }
 
 // L y = P f, y /= D, L^T x = y, u = P^T x over the whole GPU (cooperative
@@ -618,8 +791,15 @@ LdltOutcome ldlt_direct(svx_ctx* ctx, svx_op* op, double* u) {
                                                            TBLOCK, 0));
     DBuf<double> part;
     DBuf<GridBarrier> gb;
-    const bool coop_solve = coop && bps >= 1 && ctx->sm_count >= 2;
-    if (coop_solve) {
+    const bool coop_solve = coop && bps >= 1 && ctx->sm_count >= 2 && w > NARROW_BLOCKS;
+    if (w <= NARROW_BLOCKS) {
+        SVX_CUDA(cudaFuncSetAttribute(ldlt_solve_narrow_kernel,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      int(NARROW_SMEM)));
+        ldlt_solve_narrow_kernel<<<1, NBLOCK, NARROW_SMEM, st>>>(
+            n, nb, w, band.p, dfac.p, dvec.p, d_perm.p, op->f.p, y.p, u, fail.p);
+        SVX_LAUNCH_CHECK();
+    } else if (coop_solve) {
         part.alloc(ctx->pool, 2 * (size_t(w) + 1) * LT);
         gb.alloc(ctx->pool, 1);
         SVX_CUDA(cudaMemsetAsync(gb.p, 0, sizeof(GridBarrier), st));
