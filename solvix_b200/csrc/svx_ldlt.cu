@@ -65,6 +65,18 @@ __device__ __forceinline__ bool stopped(const unsigned long long* fail, int* s_f
     return *s_flag != 0;
 }
 
+// At small bandwidths the steps' kernels are launched with programmatic stream
+// serialization: a
+// kernel lets the next one start at once, and the next one waits here until it
+// has finished, so that a launch costs the wait's latency instead of a drained
+// device.  A kernel may start while the one before still writes, so what a
+// step writes is read past the L1 (__ldcg).
+constexpr int OVERLAP_BLOCKS = 24;  // up to this half-bandwidth in tiles
+__device__ __forceinline__ void step_begin() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // One thread per row r of K: its lower-triangle entries in the RCM order go
 // to the band, and max |K_rj| (the reference's row_max) to row_max[perm[r]].
 __global__ void band_fill_kernel(int64_t n, int w, const int32_t* __restrict__ perm,
@@ -133,10 +145,11 @@ ldlt_panel_kernel(int64_t J, int64_t n, int w, int wj, double* __restrict__ band
     const double* dt = band + tile_off(J, 0, w);
     double* tile = band + tile_off(J + d, d, w);
     double a[4], x[4];
+    step_begin();
 #pragma unroll
-    for (int j = 0; j < 4; ++j) a[j] = dt[r * LT + g + 8 * j];
+    for (int j = 0; j < 4; ++j) a[j] = __ldcg(dt + r * LT + g + 8 * j);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) x[q] = d <= wj ? tile[(warp + 8 * q) * LT + lane] : 0.0;
+    for (int q = 0; q < 4; ++q) x[q] = d <= wj ? __ldcg(tile + (warp + 8 * q) * LT + lane) : 0.0;
     if (threadIdx.x < LT) s_lim[threadIdx.x] = 1e-13 * fmax(row_max[J * LT + threadIdx.x], DBL_MIN);
     if (stopped(fail, &s_flag)) return;
     // Right-looking LDL^T of the tile, the whole block at once, thread (r, g)
@@ -227,8 +240,6 @@ ldlt_update_kernel(int64_t J, int w, int wj, double* __restrict__ band,
                    const double* __restrict__ panel, const unsigned long long* fail) {
     __shared__ double s_w[LT][LT + 1];  // W[r][c]
     __shared__ double s_k[LT][LT + 1];  // L[s][c]: B = L^T, column-major
-    __shared__ int s_flag;
-    if (stopped(fail, &s_flag)) return;
     int q = int(blockIdx.x), di = 1;
     while (q >= di) {
         q -= di;
@@ -241,10 +252,12 @@ ldlt_update_kernel(int64_t J, int w, int wj, double* __restrict__ band,
     double* tb = band + tile_off(J + di, di - dk, w);
     constexpr int Q = LT2 / 2 / UBLOCK;
     double2 wv[Q], lv[Q];
+    step_begin();
+    const bool stop = *(volatile const unsigned long long*)fail != NO_FAIL;
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
-        wv[q] = __ldg(wt + threadIdx.x + UBLOCK * q);
-        lv[q] = __ldg(lk + threadIdx.x + UBLOCK * q);
+        wv[q] = __ldcg(wt + threadIdx.x + UBLOCK * q);
+        lv[q] = __ldcg(lk + threadIdx.x + UBLOCK * q);
     }
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
     const int fr = lane >> 2, fc = lane & 3;
@@ -255,7 +268,9 @@ ldlt_update_kernel(int64_t J, int w, int wj, double* __restrict__ band,
         for (int sb = 0; sb < 4; ++sb)
 #pragma unroll
             for (int i = 0; i < 2; ++i)
-                tv[rb][sb][i] = tb[size_t((2 * wp + rb) * 8 + fr) * LT + sb * 8 + fc * 2 + i];
+                tv[rb][sb][i] =
+                    __ldcg(tb + size_t((2 * wp + rb) * 8 + fr) * LT + sb * 8 + fc * 2 + i);
+    if (stop) return;  // every block sees the same flag: only panel kernels set it
 #pragma unroll
     for (int q = 0; q < Q; ++q) {
         const int e = 2 * (int(threadIdx.x) + UBLOCK * q), row = e / LT, col = e % LT;
@@ -772,16 +787,31 @@ LdltOutcome ldlt_direct(svx_ctx* ctx, svx_op* op, double* u) {
         band_pad_kernel<<<1, LT, 0, st>>>(n, int64_t(rows), w, band.p, row_max.p);
         SVX_LAUNCH_CHECK();
     }
+    // Started early, the next step's blocks wait on the SMs beside this step's.
+    // The whole device time with and without, in ms: 1.69 / 1.94 at 7 tiles,
+    // 3.76 / 4.21 at 14, 10.6 / 12.1 at 22, but 21.5 / 20.6 at 34 and 43.4 /
+    // 41.6 at 47 (and 195 / 207 at 80), where a step's pairs are a few blocks an SM.
+    const unsigned early = w <= OVERLAP_BLOCKS ? 1 : 0;
+    cudaLaunchAttribute serial{};
+    serial.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    serial.val.programmaticStreamSerializationAllowed = 1;
+    auto step = [&](auto* kernel, unsigned grid, int block, auto... args) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(unsigned(block));
+        cfg.stream = st;
+        cfg.attrs = &serial;
+        cfg.numAttrs = early;
+        SVX_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+        SVX_LAUNCH_CHECK();
+    };
     for (int64_t J = 0; J < nb; ++J) {
         const int wj = int(std::min<int64_t>(w, nb - 1 - J));
-        ldlt_panel_kernel<<<unsigned(std::max(wj, 1)), LBLOCK, 0, st>>>(
-            J, n, w, wj, band.p, panel.p, dfac.p, dvec.p, row_max.p, fail.p);
-        SVX_LAUNCH_CHECK();
-        if (wj > 0) {
-            ldlt_update_kernel<<<unsigned(int64_t(wj) * (wj + 1) / 2), UBLOCK, 0, st>>>(
-                J, w, wj, band.p, panel.p, fail.p);
-            SVX_LAUNCH_CHECK();
-        }
+        step(&ldlt_panel_kernel, unsigned(std::max(wj, 1)), LBLOCK, J, n, w, wj, band.p, panel.p,
+             dfac.p, dvec.p, row_max.p, fail.p);
+        if (wj > 0)
+            step(&ldlt_update_kernel, unsigned(int64_t(wj) * (wj + 1) / 2), UBLOCK, J, w, wj,
+                 band.p, panel.p, fail.p);
     }
     // the substitutions over the whole GPU when a cooperative launch of one
     // block per SM is possible, else in one block
