@@ -51,7 +51,7 @@ sys.path.insert(0, ROOT)
 METRIC = "PCG DOF-iters/s & solves/s: mixed/batched vs FP64 at 1e-8 err; p50/p99 ms"
 UNIT = "DOF*iter/s"
 HBM_FALLBACK_GBS = 6650.0
-TRAFFIC_FILE = os.path.join(ROOT, "profiles", "pcg_smem_fp64_c3d8_160x16x16.txt")
+TRAFFIC_FILE = os.path.join(ROOT, "profiles", "brick_pcg_fp64_c3d8_160x16x16.txt")
 BATCH_TRAFFIC_FILE = os.path.join(ROOT, "profiles", "batch_pcg_fp64_plates4096_dram.txt")
 
 
@@ -133,8 +133,8 @@ def _profile_figure(path, key):
 
 
 def ncu_traffic():
-    """DRAM bytes per iteration of the shared-memory persistent PCG kernel
-    (ncu summary)."""
+    """DRAM bytes per iteration of the persistent brick PCG kernel (ncu
+    summary)."""
     return _profile_figure(TRAFFIC_FILE, "dram_bytes_per_iteration")
 
 
@@ -314,8 +314,8 @@ def run_ours(args, rank, world, local_rank):
     dof_iters = float(np.sum(iters)) * n
     value = world * dof_iters / (ms_max / 1000.0)
 
-    # roofline of the dominant kernel, the persistent PCG kernel: its
-    # algorithmic bytes per launch (CHUNK iterations) over its average
+    # roofline of the dominant kernel, the persistent PCG kernel: the
+    # algorithmic bytes of PCG on the assembled K per launch (CHUNK iterations) over its average
     # launch duration, from the PCG device time of the timed steps
     from solvix_b200.roofline import pcg_iteration_bytes, spmv_node_bytes
     # iterations per persistent launch (persistent_chunk in svx_pcg.cu)
@@ -406,17 +406,18 @@ def run_ours(args, rank, world, local_rank):
                 "d2h_bytes_per_step": int(d2h), "steps": e2e_steps,
                 "solves_per_s": world * e2e_steps / (float(e_ms.item()) / 1000.0)},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": "pcg_smem_kernel<3,8,512,1,0,1> "
-                                                 f"(FP64, {chunk} PCG iterations a launch)",
+        "roofline": {"bound": "hbm", "kernel": "brick_pcg_kernel (FP64, element by element, "
+                                                 f"{chunk} PCG iterations a launch)",
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": peak_kind,
                      "algorithmic_bytes_per_launch": int(launch_bytes),
                      "algorithmic_bytes_per_iteration": int(iter_bytes),
                      "launch_ms": float(launch_ms),
                      "traffic": traffic,
-                     "note": "K (87.7 MB in FP64 node blocks) fits the 126 MB L2; traffic "
-                             "(ncu DRAM bytes) below the algorithmic bytes is K served from "
-                             "L2 across iterations",
+                     "note": "the algorithmic bytes are an iteration's on the assembled K (87.7 "
+                             "MB), which this kernel does not read: it forms K p from the "
+                             "elements, with its constants and vectors on the chip, so the "
+                             "rate can exceed the copy peak",
                      "spmv_node_dot_alone": {
                          "launch_ms": float(kms[0]), "bytes": int(spmv_bytes),
                          "gbs": spmv_bytes / (kms[0] / 1000.0) / 1e9,
@@ -559,9 +560,9 @@ def run_batched(args, rank, world, local_rank):
                 "d2h_bytes_per_step": int(sum(8 * (f.n_dof + f.n_elem) for f in sub)),
                 "note": "svx_batch_solve from pageable host arrays, wall clock per call"},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": "batch_pcg_kernel (one CTA per member) beside "
-                                                 "batch_pcg_cluster_kernel (one 8-CTA cluster "
-                                                 "per large member), one launch each per step",
+        "roofline": {"bound": "hbm", "kernel": "FP64: resident_pcg_kernel (one cluster per plate, K "
+                                                 "in registers), one launch a size class; mixed: "
+                                                 "batch_pcg_mixed_kernel",
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": peak_kind,
                      "algorithmic_bytes_per_launch": int(bytes_alg),
@@ -1231,8 +1232,8 @@ def run_thermal(args, rank, world, local_rank):
                                           + tm.temp_value.nbytes),
                 "d2h_bytes_per_step": 8 * n},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": "pcg_persistent2_kernel<1, 16, double> and the "
-                     "assembly kernels, whole solve",
+        "roofline": {"bound": "hbm", "kernel": "spmv_node_dot and the vector kernels (CUDA graph) "
+                     "and the assembly kernels, whole solve",
                      "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_source": peak_kind, "algorithmic_bytes_per_iteration": bytes_it,
                      "note": "PCG algorithmic bytes over the whole solve's wall clock (assembly "

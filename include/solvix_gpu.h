@@ -465,8 +465,9 @@ typedef struct svx_batch_stats {
     double ms_assemble;    /* device time: all models' K1-K4 */
     double ms_solve;       /* device time of the batched PCG launch */
     double ms_stress;      /* device time of the centroid von Mises */
-    int32_t threads_per_cta;  /* autotuned CTA size of the batched PCG */
-    int32_t lanes_per_node;   /* autotuned lanes per node of its SpMV */
+    int32_t threads_per_cta;  /* CTA size of the batched PCG on the assembled K,
+                                 autotuned when members run it */
+    int32_t lanes_per_node;   /* lanes per node of its SpMV, likewise */
     int64_t total_iterations; /* sum over models */
     int64_t total_dof;        /* sum over models */
     int32_t not_converged;    /* models that missed tol within their budget
@@ -480,9 +481,11 @@ typedef struct svx_batch_stats {
  * assembled as one block-diagonal operator; one launch per size class then
  * runs every model's Jacobi-PCG with its own scalars, convergence test and
  * iteration budget (max(1000, 10 n_model) unless opts->max_iter > 0): one
- * CTA per model for the small ones and one thread-block cluster per model
- * for the large ones, largest models first.  The CTA size and lanes
- * per node are autotuned once per context and ndof, and kept.  Per model
+ * thread-block cluster of 1 to 16 CTAs per model in FP64 (plane models with
+ * K in its registers, larger solid ones element by element), one CTA or one
+ * 8-CTA cluster per model on the assembled K otherwise, largest models
+ * first.  The latter's CTA size and lanes per node are autotuned once per
+ * context and ndof, and kept.  Per model
  * outputs: u[k] (n_nodes*ndof) and von_mises[k] (n_elem), host arrays, any
  * may be NULL.  Each model is checked on its own: one that is rejected
  * (empty mesh, no constraints, a bad element found on the host or by the

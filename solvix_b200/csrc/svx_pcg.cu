@@ -14,10 +14,16 @@
 // block to finish (atomic ticket) or every block after a grid barrier sums
 // the per-block partials in index order.
 //
-// Three ways to run an iteration:
-//  * the persistent cooperative kernels (systems up to 50M nonzeros): one
+// Ways to run an iteration, the first that applies:
+//  * plane FP64 models that fit on a cluster: K in its registers
+//    (svx_resident.cu);
+//  * FP64 C3D8 models from 14,000 nodes (2,048 as batch members): element by
+//    element, in a persistent kernel on bricks of elements (svx_brick.cu) or
+//    in the graph form (svx_hex.cu);
+//  * the persistent cooperative kernels (systems whose K fits in the L2): one
 //    launch runs up to `persistent_chunk` whole iterations, its blocks
-//    meeting at bounded grid barriers;
+//    meeting at bounded grid barriers; one dof a node has its own
+//    (pcg_scalar_kernel);
 //  * the CUDA-graph form (larger systems): the standalone node-block SpMV
 //    (spmv_node_dot), update and p_update kernels, `check_every` iterations
 //    per graph launch; kernels return at once after the device status
