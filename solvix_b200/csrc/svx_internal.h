@@ -215,7 +215,11 @@ struct svx_ctx {
     // the operator element by element (svx_hex.cu, svx_brick.cu); SVX_HEX=0,
     // SVX_HEX_MIN_NODES and SVX_BRICK_MAX_ELEMS (measurements)
     int hex = 1;
-    long long hex_min_nodes = 14000, hex_batch_min_nodes = 2048;
+    long long hex_min_nodes = 14000;
+    // of a batch's members: 40 alike, on K (one CTA each) and on bricks, in ms:
+    // 45 nodes 0.58 / 0.88, 112 nodes 2.2 / 1.8, 525 nodes 33 / 8.2, 1,025
+    // nodes 68 / 9.4
+    long long hex_batch_min_nodes = 96;
     int brick_max_elems = 288;  // of a single model's brick; above: the graph form
     // elements of a brick at least, for a single model, and at most for a
     // batch's members before another CTA is added; SVX_BRICK_ELEMS and

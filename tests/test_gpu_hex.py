@@ -99,8 +99,7 @@ def test_default_context_takes_the_forms_by_size(ctx):
 
 
 def test_batch_members_of_one_to_sixteen_ctas(ctx):
-    """Members around the batch's threshold of 2,048 nodes and of every cluster
-    size; each the same alone and in the mix."""
+    """Members of every cluster size; each the same alone and in the mix."""
     sizes = [(10, 3, 3), (30, 7, 7), (32, 7, 7), (25, 16, 4), (30, 10, 10), (41, 14, 14),
              (64, 16, 16)]
     flats = [block(*s, seed=k) for k, s in enumerate(sizes)]
@@ -114,6 +113,21 @@ def test_batch_members_of_one_to_sixteen_ctas(ctx):
         alone, _ = ctx.solve_batch([flats[k]])
         assert np.array_equal(alone[0]["u"], out[k]["u"])
         assert alone[0]["iterations"] == out[k]["iterations"]
+
+
+@pytest.mark.parametrize("size", [(4, 3, 3), (5, 3, 3), (6, 3, 3), (20, 4, 4), (33, 4, 4)])
+def test_small_batch_members(ctx, size):
+    """Members about the batch's threshold of 96 nodes (80, 96, 112) and of one
+    and two CTAs (320 and 528 elements), beside a model above it and one that
+    keeps K."""
+    flats = [block(*size, seed=7), block(12, 5, 5, seed=8), with_orphan(block(*size, seed=9))]
+    out, st = ctx.solve_batch(flats)
+    assert st["not_converged"] == 0
+    for k, flat in enumerate(flats):
+        assert rel(out[k]["u"], oracle.solve_flat(flat).u) <= U_TOL, k
+    alone, _ = ctx.solve_batch(flats[:1])
+    assert np.array_equal(alone[0]["u"], out[0]["u"])
+    assert alone[0]["iterations"] == out[0]["iterations"]
 
 
 @pytest.mark.parametrize("size", [(3, 1, 1), (20, 5, 4), (48, 9, 8)])
