@@ -464,6 +464,7 @@ void device_assemble(svx_ctx* ctx, svx_op* op) {
     op->vals32q.reset();
     op->valsT.reset();
     op->vals32T.reset();
+    op->hex.stale = op->brick.stale = true;  // the element operators' constants, likewise
     apply_dirichlet(ctx, op);
     op->spmv_group = choose_spmv_group(op);
     SVX_CUDA(cudaEventRecord(ctx->ev[3], st));

@@ -795,6 +795,16 @@ size_t brick_smem(int ncap, int held, int lists, bool sm) {
 
 }  // namespace
 
+// The elements' constants, of the model as it is on the device: with the
+// bricks, and again for the first solve after every further assembly.
+void brick_constants(svx_ctx* ctx, svx_op* op) {
+    BrickOperator& B = op->brick;
+    geometry_kernel<<<unsigned((op->n_elem + 127) / 128), 128, 0, ctx->stream>>>(
+        op->n_elem, B.order.p, op->conn.p, op->xyz.p, op->youngs.p, op->poisson.p, B.geo.p);
+    SVX_LAUNCH_CHECK();
+    B.stale = false;
+}
+
 // Bricks of the members of op (one member: the whole model).  nbricks[m]:
 // bricks of member m (0: none); set to 0 for a member with a brick whose
 // nodes do not fit, a node shared by more bricks than the lists hold, or a
@@ -898,9 +908,7 @@ void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_
     entry_sort_kernel<<<dim3(members > 1 ? 16 : 256, unsigned(members)), 256, 0, st>>>(
         d_noff.p, B.entry.p, ent_n.p, fail.p, fail.p + members);
     SVX_LAUNCH_CHECK();
-    geometry_kernel<<<unsigned((op->n_elem + 127) / 128), 128, 0, st>>>(
-        op->n_elem, B.order.p, op->conn.p, op->xyz.p, op->youngs.p, op->poisson.p, B.geo.p);
-    SVX_LAUNCH_CHECK();
+    brick_constants(ctx, op);
     std::vector<int> bad(2 * size_t(members));
     SVX_CUDA(cudaMemcpyAsync(bad.data(), fail.p, sizeof(int) * bad.size(),
                              cudaMemcpyDeviceToHost, st));

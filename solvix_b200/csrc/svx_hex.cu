@@ -291,23 +291,26 @@ bool hex_applies(const svx_ctx* ctx, const svx_op* op) {
 }
 
 void hex_prepare(svx_ctx* ctx, svx_op* op) {
-    if (op->hex.rdet.p) return;
-    cudaStream_t st = ctx->stream;
     HexOperator& h = op->hex;
+    if (h.slot.p && !h.stale) return;
+    cudaStream_t st = ctx->stream;
     const Pattern& P = op->pat;
-    h.rdet.alloc(ctx->pool, size_t(op->n_elem) * 8);
-    h.lame.alloc(ctx->pool, size_t(op->n_elem));
-    h.x4.alloc(ctx->pool, size_t(op->n_nodes) * 4);
-    h.slot.alloc(ctx->pool, size_t(op->n_nodes) * std::max(P.max_slots, 1));
+    if (!h.slot.p) {
+        h.rdet.alloc(ctx->pool, size_t(op->n_elem) * 8);
+        h.lame.alloc(ctx->pool, size_t(op->n_elem));
+        h.x4.alloc(ctx->pool, size_t(op->n_nodes) * 4);
+        h.slot.alloc(ctx->pool, size_t(op->n_nodes) * std::max(P.max_slots, 1));
+        hex_slots_kernel<<<blocks(op->n_nodes, NB), NB, 0, st>>>(
+            op->n_nodes, op->n_elem, P.max_slots, P.slot_ptr.p, P.slot_elem.p, P.slot_local.p,
+            h.slot.p);
+        SVX_LAUNCH_CHECK();
+    }
     hex_setup_kernel<<<blocks(op->n_elem, HB), HB, 0, st>>>(
         op->n_elem, op->conn.p, op->xyz.p, op->youngs.p, op->poisson.p, h.rdet.p, h.lame.p);
     SVX_LAUNCH_CHECK();
-    hex_slots_kernel<<<blocks(op->n_nodes, NB), NB, 0, st>>>(
-        op->n_nodes, op->n_elem, P.max_slots, P.slot_ptr.p, P.slot_elem.p, P.slot_local.p,
-        h.slot.p);
-    SVX_LAUNCH_CHECK();
     pad_rows_kernel<<<blocks(op->n_nodes, NB), NB, 0, st>>>(op->n_nodes, op->xyz.p, h.x4.p);
     SVX_LAUNCH_CHECK();
+    h.stale = false;
 }
 
 void HexWork::alloc(svx_ctx* ctx, const svx_op* op) {

@@ -295,6 +295,9 @@ struct HexOperator {
     DBuf<double2> lame;   // [n_elem] Lame constants / 512
     DBuf<double> x4;      // [n_nodes][4] coordinates
     DBuf<uint32_t> slot;  // [max_slots][n_nodes] force offsets of a node's slots
+    // an assembly has run since the constants (not the slots, which like the
+    // pattern depend on the connectivity alone) were formed
+    bool stale = false;
 };
 
 // The bricks of C3D8 models (svx_brick.cu).
@@ -317,6 +320,7 @@ struct BrickView {
 struct BrickOperator {
     int bricks = 0, ncap = 0, held = 0, lists = 0;
     int state = 0;     // single models: 0 not built, 1 built, -1 does not fit
+    bool stale = false;  // geo is older than the last assembly (the lists are not)
     DBuf<int32_t> elem0, elem1, member, chunk0, order, count, node, ccount, member_brick;
     DBuf<uint16_t> lconn, cnode, ref;
     DBuf<uint32_t> entry;
@@ -511,6 +515,7 @@ struct BrickWork {
     DBuf<GridBarrier> gb;
     void alloc(svx_ctx* ctx, const svx_op* op, bool single);
 };
+void brick_constants(svx_ctx* ctx, svx_op* op);  // geo, from the model on the device
 void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_t>& node_off,
                  const std::vector<int64_t>& elem_off, std::vector<int>& nbricks);
 void brick_grid_launch(svx_ctx* ctx, const svx_op* op, BrickWork& w, double* u, double* r,

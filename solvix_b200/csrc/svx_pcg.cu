@@ -3207,6 +3207,7 @@ static void wire_hex_form(svx_ctx* ctx, svx_op* op, PcgRun<double, double, doubl
         op->brick.state = nbricks[0] > 0 ? 1 : -1;
     }
     if (op->brick.state > 0) {
+        if (op->brick.stale) brick_constants(ctx, op);
         brick.alloc(ctx, op, true);
         run.brick = &brick;
         return;
