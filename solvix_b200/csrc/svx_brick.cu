@@ -61,14 +61,17 @@ constexpr int SHARE = 8;            // bricks that may touch a node
 
 // ------------------------------------------------------------ building
 // The layer of every element along its member's longest side; one CTA a
-// member.
+// member of the list (those with bricks: a batch may have any number of
+// others, and more members than a grid's y or z dimension).
 __global__ void __launch_bounds__(1024)
-layer_kernel(const int64_t* __restrict__ node_off, const int64_t* __restrict__ elem_off,
-             const int32_t* __restrict__ conn, const double* __restrict__ xyz,
-             uint16_t* __restrict__ layer, int32_t* __restrict__ hist) {
+layer_kernel(const int32_t* __restrict__ list, const int64_t* __restrict__ node_off,
+             const int64_t* __restrict__ elem_off, const int32_t* __restrict__ conn,
+             const double* __restrict__ xyz, uint16_t* __restrict__ layer,
+             int32_t* __restrict__ hist) {
     __shared__ double box[6][32];
-    const int64_t n0 = node_off[blockIdx.x], n1 = node_off[blockIdx.x + 1];
-    const int64_t e0 = elem_off[blockIdx.x], e1 = elem_off[blockIdx.x + 1];
+    const int member = list[blockIdx.x];
+    const int64_t n0 = node_off[member], n1 = node_off[member + 1];
+    const int64_t e0 = elem_off[member], e1 = elem_off[member + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double b[6];
 #pragma unroll
@@ -115,37 +118,42 @@ layer_kernel(const int64_t* __restrict__ node_off, const int64_t* __restrict__ e
     }
 }
 
-// Elements by layer, in index order within a layer: one CTA per layer and
-// member.
+// Elements by layer, in index order within a layer: gridDim.y CTAs a member
+// of the list share its layers (a CTA a layer for a single model; 16 a member
+// of a batch, where most of 1,024 would find an empty layer).
 __global__ void __launch_bounds__(256)
-layer_order_kernel(const int64_t* __restrict__ elem_off, const uint16_t* __restrict__ layer,
-                   const int32_t* __restrict__ hist, int32_t* __restrict__ order) {
+layer_order_kernel(const int32_t* __restrict__ list, const int64_t* __restrict__ elem_off,
+                   const uint16_t* __restrict__ layer, const int32_t* __restrict__ hist,
+                   int32_t* __restrict__ order) {
     __shared__ int sums[8], base;
-    const int L = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int32_t* h = hist + int64_t(blockIdx.y) * BRICK_LAYERS;
-    if (h[L] == 0) return;
-    const int64_t e0 = elem_off[blockIdx.y], e1 = elem_off[blockIdx.y + 1];
-    if (threadIdx.x == 0) base = 0;
-    __syncthreads();
-    int before = 0;
-    for (int k = threadIdx.x; k < L; k += 256) before += h[k];
-    if (before) atomicAdd(&base, before);
-    __syncthreads();
-    int at = base;
-    for (int64_t c = e0; c < e1; c += 256) {
-        const int64_t e = c + threadIdx.x;
-        const bool in = e < e1 && layer[e] == L;
-        const unsigned m = __ballot_sync(0xffffffffu, in);
-        if (lane == 0) sums[warp] = __popc(m);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int member = list[blockIdx.x];
+    const int32_t* h = hist + int64_t(blockIdx.x) * BRICK_LAYERS;
+    const int64_t e0 = elem_off[member], e1 = elem_off[member + 1];
+    for (int L = blockIdx.y; L < BRICK_LAYERS; L += gridDim.y) {
+        if (h[L] == 0) continue;
+        if (threadIdx.x == 0) base = 0;
         __syncthreads();
-        int pos = at, all = 0;
-        for (int w = 0; w < 8; ++w) {
-            if (w < warp) pos += sums[w];
-            all += sums[w];
+        int before = 0;
+        for (int k = threadIdx.x; k < L; k += 256) before += h[k];
+        if (before) atomicAdd(&base, before);
+        __syncthreads();
+        int at = base;
+        for (int64_t c = e0; c < e1; c += 256) {
+            const int64_t e = c + threadIdx.x;
+            const bool in = e < e1 && layer[e] == L;
+            const unsigned m = __ballot_sync(0xffffffffu, in);
+            if (lane == 0) sums[warp] = __popc(m);
+            __syncthreads();
+            int pos = at, all = 0;
+            for (int w = 0; w < 8; ++w) {
+                if (w < warp) pos += sums[w];
+                all += sums[w];
+            }
+            if (in) order[e0 + pos + __popc(m & ((1u << lane) - 1u))] = int32_t(e);
+            at += all;
+            __syncthreads();
         }
-        if (in) order[e0 + pos + __popc(m & ((1u << lane) - 1u))] = int32_t(e);
-        at += all;
-        __syncthreads();
     }
 }
 
@@ -275,17 +283,19 @@ brick_build_kernel(BrickView b, const int32_t* __restrict__ conn, int32_t* ent_n
 }
 
 // Every node's entries in ascending brick order, and how many nodes more than
-// three bricks share; gridDim.y members.
-__global__ void entry_sort_kernel(const int64_t* __restrict__ node_off,
+// three bricks share; gridDim.y CTAs a member of the list.
+__global__ void entry_sort_kernel(const int32_t* __restrict__ list,
+                                  const int64_t* __restrict__ node_off,
                                   uint32_t* __restrict__ entry,
                                   const int32_t* __restrict__ ent_n, int* __restrict__ fail,
                                   int* __restrict__ crowded) {
-    const int64_t n1 = node_off[blockIdx.y + 1];
-    for (int64_t i = node_off[blockIdx.y] + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-         i < n1; i += int64_t(gridDim.x) * blockDim.x) {
+    const int member = list[blockIdx.x];
+    const int64_t n1 = node_off[member + 1];
+    for (int64_t i = node_off[member] + int64_t(blockIdx.y) * blockDim.x + threadIdx.x;
+         i < n1; i += int64_t(gridDim.y) * blockDim.x) {
         const int n = min(ent_n[i], SHARE);
-        if (n == 0) fail[blockIdx.y] = 1;
-        if (n > 3) atomicAdd(&crowded[blockIdx.y], 1);
+        if (n == 0) fail[member] = 1;
+        if (n > 3) atomicAdd(&crowded[member], 1);
         uint32_t* e = entry + i * SHARE;
         for (int a = 1; a < n; ++a) {
             const uint32_t v = e[a];
@@ -297,36 +307,36 @@ __global__ void entry_sort_kernel(const int64_t* __restrict__ node_off,
     }
 }
 
-// The elements' constants, in brick order.
-__global__ void geometry_kernel(int64_t n_elem, const int32_t* __restrict__ order,
-                                const int32_t* __restrict__ conn,
-                                const double* __restrict__ xyz,
-                                const double* __restrict__ youngs,
-                                const double* __restrict__ poisson, double* __restrict__ geo) {
-    const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (k >= n_elem) return;
-    const int64_t e = order[k];
-    double x[8][3];
+// The elements' constants, in brick order: one CTA a brick.
+__global__ void __launch_bounds__(CH)
+geometry_kernel(BrickView b, int64_t n_elem, const int32_t* __restrict__ conn,
+                const double* __restrict__ xyz, const double* __restrict__ youngs,
+                const double* __restrict__ poisson, double* __restrict__ geo) {
+    for (int64_t k = b.elem0[blockIdx.x] + int64_t(threadIdx.x); k < b.elem1[blockIdx.x];
+         k += CH) {
+        const int64_t e = b.order[k];
+        double x[8][3];
 #pragma unroll
-    for (int a = 0; a < 8; ++a) {
-        const int64_t nd = conn[8 * e + a];
+        for (int a = 0; a < 8; ++a) {
+            const int64_t nd = conn[8 * e + a];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) x[a][c] = xyz[3 * nd + c];
+            for (int c = 0; c < 3; ++c) x[a][c] = xyz[3 * nd + c];
+        }
+        HexModes X(x);
+        const double* m = X.c1;
+#pragma unroll
+        for (int q = 0; q < 21; ++q) geo[q * n_elem + k] = m[q];
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+            double J[3][3];
+            X.gradient(g, J);
+            geo[(21 + g) * n_elem + k] = 1.0 / hex_det(J);
+        }
+        double lam, mu;
+        hex_lame(youngs[e], poisson[e], lam, mu);
+        geo[29 * n_elem + k] = lam;
+        geo[30 * n_elem + k] = mu;
     }
-    HexModes X(x);
-    const double* m = X.c1;
-#pragma unroll
-    for (int q = 0; q < 21; ++q) geo[q * n_elem + k] = m[q];
-#pragma unroll
-    for (int g = 0; g < 8; ++g) {
-        double J[3][3];
-        X.gradient(g, J);
-        geo[(21 + g) * n_elem + k] = 1.0 / hex_det(J);
-    }
-    double lam, mu;
-    hex_lame(youngs[e], poisson[e], lam, mu);
-    geo[29 * n_elem + k] = lam;
-    geo[30 * n_elem + k] = mu;
 }
 
 // ------------------------------------------------------------ solving
@@ -799,8 +809,8 @@ size_t brick_smem(int ncap, int held, int lists, bool sm) {
 // bricks, and again for the first solve after every further assembly.
 void brick_constants(svx_ctx* ctx, svx_op* op) {
     BrickOperator& B = op->brick;
-    geometry_kernel<<<unsigned((op->n_elem + 127) / 128), 128, 0, ctx->stream>>>(
-        op->n_elem, B.order.p, op->conn.p, op->xyz.p, op->youngs.p, op->poisson.p, B.geo.p);
+    geometry_kernel<<<B.bricks, CH, 0, ctx->stream>>>(B.view(), op->n_elem, op->conn.p, op->xyz.p,
+                                                      op->youngs.p, op->poisson.p, B.geo.p);
     SVX_LAUNCH_CHECK();
     B.stale = false;
 }
@@ -814,7 +824,7 @@ void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_
     BrickOperator& B = op->brick;
     cudaStream_t st = ctx->stream;
     const int members = int(nbricks.size());
-    std::vector<int32_t> e0, e1, mb(1, 0), c0, bm;
+    std::vector<int32_t> e0, e1, mb(1, 0), c0, bm, list;  // list: the members with bricks
     int chunks = 0, most = 0;
     for (int m = 0; m < members; ++m)
         if (nbricks[m])
@@ -830,6 +840,7 @@ void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_
             e1.push_back(int32_t(z));
             bm.push_back(m);
         }
+        if (nbricks[m]) list.push_back(m);
         mb.push_back(int32_t(c0.size()));
     }
     const int bricks = int(c0.size());
@@ -857,12 +868,14 @@ void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_
     B.bricks = bricks;
     DBuf<int64_t> d_noff, d_eoff;
     DBuf<uint16_t> layer;
-    DBuf<int32_t> hist, ent_n;
+    DBuf<int32_t> hist, ent_n, d_list;
     DBuf<int> fail;
+    const unsigned listed = unsigned(list.size());
     d_noff.alloc(ctx->pool, members + 1);
     d_eoff.alloc(ctx->pool, members + 1);
     layer.alloc(ctx->pool, size_t(op->n_elem));
-    hist.alloc(ctx->pool, size_t(members) * BRICK_LAYERS);
+    d_list.alloc(ctx->pool, listed);
+    hist.alloc(ctx->pool, size_t(listed) * BRICK_LAYERS);
     ent_n.alloc(ctx->pool, size_t(op->n_nodes));
     fail.alloc(ctx->pool, 2 * size_t(members));  // and the nodes many bricks share
     B.order.alloc(ctx->pool, size_t(op->n_elem));
@@ -885,19 +898,20 @@ void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_
     };
     up(d_noff, node_off);
     up(d_eoff, elem_off);
+    up(d_list, list);
     up(B.elem0, e0);
     up(B.elem1, e1);
     up(B.member, bm);
     up(B.chunk0, c0);
     up(B.member_brick, mb);
-    SVX_CUDA(cudaMemsetAsync(hist.p, 0, sizeof(int32_t) * size_t(members) * BRICK_LAYERS, st));
+    SVX_CUDA(cudaMemsetAsync(hist.p, 0, sizeof(int32_t) * size_t(listed) * BRICK_LAYERS, st));
     SVX_CUDA(cudaMemsetAsync(ent_n.p, 0, sizeof(int32_t) * size_t(op->n_nodes), st));
     SVX_CUDA(cudaMemsetAsync(fail.p, 0, sizeof(int) * 2 * size_t(members), st));
-    layer_kernel<<<members, 1024, 0, st>>>(d_noff.p, d_eoff.p, op->conn.p, op->xyz.p, layer.p,
-                                           hist.p);
+    layer_kernel<<<listed, 1024, 0, st>>>(d_list.p, d_noff.p, d_eoff.p, op->conn.p, op->xyz.p,
+                                          layer.p, hist.p);
     SVX_LAUNCH_CHECK();
-    layer_order_kernel<<<dim3(BRICK_LAYERS, unsigned(members)), 256, 0, st>>>(d_eoff.p, layer.p,
-                                                                            hist.p, B.order.p);
+    layer_order_kernel<<<dim3(listed, single ? BRICK_LAYERS : 16), 256, 0, st>>>(
+        d_list.p, d_eoff.p, layer.p, hist.p, B.order.p);
     SVX_LAUNCH_CHECK();
     const size_t bsm = size_t(SORT_BRICK + ncap) * 4;
     SVX_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(&brick_build_kernel),
@@ -905,8 +919,8 @@ void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_
                                   int((SORT_BRICK + 4096) * 4)));
     brick_build_kernel<<<bricks, BT, bsm, st>>>(B.view(), op->conn.p, ent_n.p, fail.p);
     SVX_LAUNCH_CHECK();
-    entry_sort_kernel<<<dim3(members > 1 ? 16 : 256, unsigned(members)), 256, 0, st>>>(
-        d_noff.p, B.entry.p, ent_n.p, fail.p, fail.p + members);
+    entry_sort_kernel<<<dim3(listed, single ? 256 : 16), 256, 0, st>>>(
+        d_list.p, d_noff.p, B.entry.p, ent_n.p, fail.p, fail.p + members);
     SVX_LAUNCH_CHECK();
     brick_constants(ctx, op);
     std::vector<int> bad(2 * size_t(members));
