@@ -216,10 +216,13 @@ struct svx_ctx {
     // SVX_HEX_MIN_NODES and SVX_BRICK_MAX_ELEMS (measurements)
     int hex = 1;
     long long hex_min_nodes = 14000;
-    // of a batch's members: 40 alike, on K (one CTA each) and on bricks, in ms:
-    // 45 nodes 0.58 / 0.88, 112 nodes 2.2 / 1.8, 525 nodes 33 / 8.2, 1,025
-    // nodes 68 / 9.4
-    long long hex_batch_min_nodes = 96;
+    // of a batch's members, alone or among any others (a member's bits must not
+    // depend on its batch).  On K (one CTA each) and on bricks, in ms, for 40
+    // and 4,000 alike: 117 nodes 1.2 / 1.1 and 19.0 / 26.9, 144 nodes 0.98 /
+    // 0.86 and 19.5 / 22.1, 176 nodes 1.6 / 1.1 and 28.9 / 27.5, 189 nodes 3.0 /
+    // 1.8 and 55 / 47, 208 nodes 2.9 / 1.2 and 50 / 32, 525 nodes 16.0 / 4.8 and
+    // 264 / 126: below, K's CTAs share an SM, where a brick has one to itself.
+    long long hex_batch_min_nodes = 180;
     int brick_max_elems = 288;  // of a single model's brick; above: the graph form
     // elements of a brick at least, for a single model, and at most for a
     // batch's members before another CTA is added; SVX_BRICK_ELEMS and

@@ -17,7 +17,7 @@
 // Ways to run an iteration, the first that applies:
 //  * plane FP64 models that fit on a cluster: K in its registers
 //    (svx_resident.cu);
-//  * FP64 C3D8 models from 14,000 nodes (96 as batch members): element by
+//  * FP64 C3D8 models from 14,000 nodes (180 as batch members): element by
 //    element, in a persistent kernel on bricks of elements (svx_brick.cu) or
 //    in the graph form (svx_hex.cu);
 //  * the persistent cooperative kernels (systems whose K fits in the L2): one
