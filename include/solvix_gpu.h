@@ -608,6 +608,17 @@ int svx_op_time_kernels(svx_op_t* op, int reps, double* ms4);
  * time-out to its caller) and *error_flag (1 = the flag was raised). */
 int svx_diag_barrier_timeout(int device, long long spins, int* returned_ok, int* error_flag);
 
+/* No counterpart in the reference.  The same for the waits between the CTAs
+ * of the cluster that solves a plane model: solves the operator with one
+ * thing wrong in an early iteration, and waits that run out after wait_us
+ * microseconds (1..10^6).  fault 0, 1: one CTA does not send its part of
+ * p.Kp, of r.r and r.z; 2, 3: a third of one CTA's threads take that wait to
+ * have run out although the sums came, so its threads disagree.  The kernel
+ * ends by itself in every case and the call returns what a solve would,
+ * SVX_CUDA_ERROR with the stall's text; the context stays usable.
+ * SVX_BAD_ARGUMENT: no operator that more than one CTA solves. */
+int svx_diag_resident_stall(svx_op_t* op, int fault, long long wait_us, svx_error_t* err);
+
 /* ---- PCG without device allocation ---------------------------------- */
 /* Largest system (rows) svx_pcg_solve_noalloc accepts. */
 #define SVX_NOALLOC_MAX_DOF 262144

@@ -299,6 +299,7 @@ SIGNATURES = {
     "svx_launch_count": (C.c_int64, []),
     "svx_diag_barrier_timeout": (C.c_int, [C.c_int, C.c_longlong, C.POINTER(C.c_int),
                                            C.POINTER(C.c_int)]),
+    "svx_diag_resident_stall": (C.c_int, [_VP, C.c_int, C.c_longlong, C.POINTER(SvxError)]),
     "svx_op_time_kernels": (C.c_int, [_VP, C.c_int, c_double_p]),
     "svx_pcg_solve_noalloc": (C.c_int, [C.c_int64, _VP, _VP, _VP, _VP, C.c_double, C.c_int64,
                                         _VP, c_int64_p, c_double_p, _VP]),

@@ -1188,6 +1188,19 @@ int svx_op_reassemble(svx_op_t* op, svx_error_t* err) {
     });
 }
 
+int svx_diag_resident_stall(svx_op_t* op, int fault, long long wait_us, svx_error_t* err) {
+    if (!op || fault < 0 || fault > 3 || wait_us <= 0 || wait_us > 1000000)
+        return SVX_BAD_ARGUMENT;
+    svx_ctx* ctx = op->ctx;
+    return guarded(ctx, err, [&]() -> int {
+        refuse_mass(op, "it is not solved");
+        SVX_CUDA(cudaSetDevice(ctx->device));
+        resident_stall_diag(ctx, op, fault, wait_us * 1000);
+        clear_error(err);
+        return SVX_OK;
+    });
+}
+
 int svx_op_free(svx_op_t* op) {
     if (!op) return SVX_OK;
     cudaSetDevice(op->ctx->device);

@@ -543,11 +543,15 @@ void resident_order(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int
                     std::vector<int64_t>& span);
 bool resident_shape(const svx_ctx* ctx, int64_t n, int64_t span, bool single,
                     ResidentShape* out);
-// `count` members of op, one cluster each; all pointers on the device.
+// `count` members of op, one cluster each; all pointers on the device.  fault
+// >= 0: the diagnostic form, whose waits run out after wait_ns (clusters only).
 void resident_pcg(svx_ctx* ctx, const svx_op* op, const ResidentShape& shape, bool single, cudaStream_t st,
                   int count, const int32_t* order, const int64_t* node_off, const double* tol,
                   const int64_t* max_iter, int64_t* out_it, double* out_res,
-                  int32_t* out_status, double* u);
+                  int32_t* out_status, double* u, int fault = -1, long long wait_ns = 0);
+// Throws the stall's error if the diagnostic form of a kept plane operator's
+// solve reports it, as a solve would.
+void resident_stall_diag(svx_ctx* ctx, svx_op* op, int fault, long long wait_ns);
 
 void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& node_off,
                const std::vector<int64_t>& elem_off,

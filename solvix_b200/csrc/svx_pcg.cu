@@ -3166,7 +3166,8 @@ static const char* const RESIDENT_STALL_TEXT =
 
 // One plane model on the chip-resident cluster kernel (svx_resident.cu).
 static PcgResult pcg_resident(svx_ctx* ctx, svx_op* op, const ResidentShape& shape, double tol,
-                              long long max_iter, double* u_dev) {
+                              long long max_iter, double* u_dev, int fault = -1,
+                              long long wait_ns = 0) {
     struct Slot {
         int64_t off[2], max_iter, it;
         double tol, res;
@@ -3181,7 +3182,7 @@ static PcgResult pcg_resident(svx_ctx* ctx, svx_op* op, const ResidentShape& sha
     SVX_CUDA(cudaMemcpyAsync(d.p, h, sizeof(Slot), cudaMemcpyHostToDevice, st));
     SVX_CUDA(cudaEventRecord(ctx->ev[0], st));
     resident_pcg(ctx, op, shape, true, st, 1, nullptr, d.p->off, &d.p->tol, &d.p->max_iter, &d.p->it,
-                 &d.p->res, &d.p->status, u_dev);
+                 &d.p->res, &d.p->status, u_dev, fault, wait_ns);
     SVX_CUDA(cudaEventRecord(ctx->ev[1], st));
     SVX_CUDA(cudaMemcpyAsync(h, d.p, sizeof(Slot), cudaMemcpyDeviceToHost, st));
     SVX_CUDA(cudaStreamSynchronize(st));
@@ -3189,6 +3190,26 @@ static PcgResult pcg_resident(svx_ctx* ctx, svx_op* op, const ResidentShape& sha
     SVX_CUDA(cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]));
     if (h->status == RESIDENT_STALLED) throw ModelFail{SVX_CUDA_ERROR, 0, -1, RESIDENT_STALL_TEXT};
     return PcgResult{h->status, h->it, h->res, ms};
+}
+
+// The cluster shape of a plane operator's FP64 solve; false: another form.
+static bool resident_single_shape(svx_ctx* ctx, svx_op* op, ResidentShape* shape) {
+    if (op->slot_span < 0) {
+        std::vector<int64_t> span{0};
+        resident_order(ctx, op, true, {0, op->n_nodes}, span);
+        op->slot_span = span[0];
+    }
+    return resident_shape(ctx, op->n_nodes, op->slot_span, true, shape);
+}
+
+void resident_stall_diag(svx_ctx* ctx, svx_op* op, int fault, long long wait_ns) {
+    ResidentShape shape;
+    if (op->ndof != 2 || op->n_nodes >= RESIDENT_MAX_NODES || op->pat.max_deg > RESIDENT_MAX_DEG ||
+        !resident_single_shape(ctx, op, &shape) || shape.ctas < 2)
+        throw ModelFail{SVX_BAD_ARGUMENT, 0, -1, "not an operator that a cluster solves"};
+    DBuf<double> u;
+    u.alloc(ctx->pool, op->n);
+    pcg_resident(ctx, op, shape, 1e-10, 1000, u.p, fault, wait_ns);
 }
 
 // Gives an FP64 run of a C3D8 model its element-by-element form, where it
@@ -3249,13 +3270,8 @@ PcgResult pcg_fp64(svx_ctx* ctx, svx_op* op, double tol, long long max_iter, int
     if (op->ndof == 2 && op->n_nodes < RESIDENT_MAX_NODES && ctx->resident && ctx->pcg_smem &&
         op->pat.max_deg <= RESIDENT_MAX_DEG && max_iter <= RESIDENT_MAX_ITER &&
         !use_graph_form(ctx, op)) {
-        if (op->slot_span < 0) {
-            std::vector<int64_t> span{0};
-            resident_order(ctx, op, true, {0, op->n_nodes}, span);
-            op->slot_span = span[0];
-        }
         ResidentShape shape;
-        if (resident_shape(ctx, op->n_nodes, op->slot_span, true, &shape))
+        if (resident_single_shape(ctx, op, &shape))
             return pcg_resident(ctx, op, shape, tol, max_iter, u_dev);
     }
     if (check_every <= 0) check_every = auto_check_every(n, op->pat.nnz);

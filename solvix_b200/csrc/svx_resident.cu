@@ -73,6 +73,8 @@ struct ResidentArgs {
     double* out_res;
     int32_t* out_status;
     int window_cap;            // nodes a CTA's window may hold
+    unsigned long long wait_ns;  // a wait between CTAs runs out after this long
+    int fault;                 // DIAG: which exchange goes wrong, and how
 };
 
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
@@ -104,7 +106,8 @@ __device__ __forceinline__ void bar_expect(unsigned bar, unsigned bytes) {
                  : "memory");
 }
 // Waits for the phase of the given parity; false when it has not completed
-// within two seconds.
+// within wait_ns.  The verdict is this thread's alone: the phase may complete
+// between two threads' limits, so nobody acts on it before the CTA has voted.
 constexpr unsigned long long WAIT_NS = 2000000000ull;
 __device__ __forceinline__ bool bar_done(unsigned bar, unsigned parity) {
     unsigned done;
@@ -115,21 +118,25 @@ __device__ __forceinline__ bool bar_done(unsigned bar, unsigned parity) {
         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     return done != 0;
 }
-__device__ __noinline__ bool bar_wait_long(unsigned bar, unsigned parity) {
+__device__ __noinline__ bool bar_wait_long(unsigned bar, unsigned parity,
+                                           unsigned long long wait_ns) {
     unsigned long long start, now;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(start));
     do {
+        // polled after the clock is read: a thread that was switched out for
+        // longer than the limit still looks once more
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
         for (int k = 0; k < 64; ++k)
             if (bar_done(bar, parity)) return true;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
-    } while (now - start < WAIT_NS);
+    } while (now - start < wait_ns);
     return false;
 }
-__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
+__device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity,
+                                         unsigned long long wait_ns) {
 #pragma unroll 1
     for (int k = 0; k < 64; ++k)
         if (bar_done(bar, parity)) return true;
-    return bar_wait_long(bar, parity);
+    return bar_wait_long(bar, parity, wait_ns);
 }
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
@@ -159,7 +166,10 @@ struct Inbox {
 // T: most threads of a CTA.  512 leaves a thread 128 registers, so a batch
 // also runs two CTAs of 256 on an SM; a single solve's CTAs of up to 256
 // threads have their SM to themselves and take all the registers they want.
-template <bool SINGLE, int T>
+// DIAG: an early iteration's exchange a.fault & 1 (0: A, 1: B) goes wrong in
+// CTA 1, which drops its sums (a.fault < 2) or takes the wait of every third
+// thread to have run out (2, 3).
+template <bool SINGLE, int T, bool DIAG = false>
 __global__ void __launch_bounds__(T, 1) resident_pcg_kernel(ResidentArgs a) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ __align__(16) Inbox box;
@@ -284,6 +294,9 @@ __global__ void __launch_bounds__(T, 1) resident_pcg_kernel(ResidentArgs a) {
     // p.Kp of the model from the threads' terms: warp sums, their sum in
     // warp 0, one message to every CTA (an exchange costs about 7 cycles for
     // every message a CTA receives), and their sum in every warp
+    auto faulty = [&](unsigned parity, int fault) {
+        return DIAG && parity == 1u && rank == 1u && a.fault == fault;
+    };
     auto reduce_a = [&](double x, unsigned parity, double& total) -> bool {
         x = lane_sum(x);
         if (lane == 0) warp_a[warp] = x;
@@ -294,23 +307,29 @@ __global__ void __launch_bounds__(T, 1) resident_pcg_kernel(ResidentArgs a) {
         } else {
             if (warp == 0) {
                 x = lane_sum(lane < warps ? warp_a[lane] : 0.0);
-                if (sends)
+                if (sends && !faulty(parity, 0))
                     send(peer_box + unsigned(offsetof(Inbox, part_a)) + rank * 8, x,
                          peer_box + unsigned(offsetof(Inbox, bar_a)));
             }
-            const bool ok = bar_wait(bar_a, parity);
+            const bool ok = bar_wait(bar_a, parity, a.wait_ns);
             __syncwarp();
             total = lane_sum(lane < int(ctas) ? box.part_a[lane] : 0.0);
-            return ok;
+            return ok && !(faulty(parity, 2) && t % 3 == 0);
         }
     };
-    // r.r and r.z of the model
-    auto reduce_b = [&](double x, double y, unsigned parity, double& tx, double& ty) -> bool {
+    // r.r and r.z of the model, and the vote on the wait before (ok): the CTA
+    // sends its sums, which let the others go on, only if all of its threads
+    // came through.  Returns what ends the solve here, the same in every
+    // thread: a wait that ran out, or p.Kp <= 0 (broke; all threads have the
+    // same p.Kp when none of their waits ran out).
+    auto reduce_b = [&](double x, double y, bool& ok, bool broke, unsigned parity, double& tx,
+                        double& ty) -> int {
         double v = lane_sum_pair(x, y, lane);
         if ((lane & 15) == 0) warp_b[2 * warp + (lane >> 4)] = v;
-        __syncthreads();
+        if constexpr (SINGLE) __syncthreads();
+        else if (__syncthreads_or(!ok)) return RESIDENT_STALLED;
+        if (broke) return PCG_BREAKDOWN;
         double2 w = make_double2(0.0, 0.0);
-        bool ok = true;
         if (SINGLE || warp == 0) {
             if (lane < warps) w = make_double2(warp_b[2 * lane], warp_b[2 * lane + 1]);
         }
@@ -318,17 +337,17 @@ __global__ void __launch_bounds__(T, 1) resident_pcg_kernel(ResidentArgs a) {
             if (warp == 0) {
                 v = lane_sum_pair(w.x, w.y, lane);
                 const double other = __shfl_xor_sync(0xffffffffu, v, 16);
-                if (sends)
+                if (sends && !faulty(parity, 1))
                     send2(peer_box + unsigned(offsetof(Inbox, part_b)) + rank * 16, v, other,
                           peer_box + unsigned(offsetof(Inbox, bar_b)));
             }
-            ok = bar_wait(bar_b, parity);
+            ok = bar_wait(bar_b, parity, a.wait_ns) && !(faulty(parity, 3) && t % 3 == 0);
             __syncwarp();
             w = lane < int(ctas) ? box.part_b[lane] : make_double2(0.0, 0.0);
         }
         tx = lane_sum(w.x);
         ty = lane_sum(w.y);
-        return ok;
+        return PCG_RUNNING;
     };
     const double tl = a.tol[inst];
     const int mi = int(a.max_iter[inst]);  // at most RESIDENT_MAX_ITER
@@ -343,7 +362,8 @@ __global__ void __launch_bounds__(T, 1) resident_pcg_kernel(ResidentArgs a) {
         push(z);
     }
     double rr, rz;
-    bool ok = reduce_b(lrr, lrz, 0, rr, rz);
+    bool ok = true;  // this thread's last wait
+    reduce_b(lrr, lrz, ok, false, 0, rr, rz);
     const double bnorm = sqrt(rr);
     // above this r.r, sqrt(r.r) / ||f|| cannot round to tol or less, so the
     // root and the quotient are left to the last iterations
@@ -352,8 +372,11 @@ __global__ void __launch_bounds__(T, 1) resident_pcg_kernel(ResidentArgs a) {
     int it = 0;
     int status = (bnorm == 0.0) ? PCG_CONVERGED : PCG_RUNNING;
     double beta = 0.0;
-    while (status == PCG_RUNNING && ok) {
-        if (!SINGLE && t == 0) {
+    for (;;) {
+        if (SINGLE && status != PCG_RUNNING) break;
+        // (a thread whose wait ran out has seen no phase end, so it must not
+        // open the next one)
+        if (!SINGLE && t == 0 && ok) {
             bar_expect(bar_a, bytes_a);
             bar_expect(bar_b, bytes_b);
         }
@@ -368,7 +391,14 @@ __global__ void __launch_bounds__(T, 1) resident_pcg_kernel(ResidentArgs a) {
                 const double2 zz = zw[w], pp = pw[w];
                 pw[w] = make_double2(__fma_rn(beta, pp.x, zz.x), __fma_rn(beta, pp.y, zz.y));
             }
-        __syncthreads();
+        if constexpr (SINGLE) {
+            __syncthreads();
+        } else {
+            // the vote on exchange B's wait; its outcome stands only now (the
+            // one p too many at the end costs less than a barrier of its own)
+            if (__syncthreads_or(!ok)) status = RESIDENT_STALLED;
+            if (status != PCG_RUNNING) break;
+        }
         // q = K p on the own rows, p.q
         // (two chains a row, over the first five and the last four neighbours)
         double2 qc[2] = {};
@@ -385,15 +415,11 @@ __global__ void __launch_bounds__(T, 1) resident_pcg_kernel(ResidentArgs a) {
         double pap;
         ok = reduce_a(p.x * q.x + p.y * q.y, unsigned(it) & 1u, pap);
         it += 1;
-        if (!ok) break;
-        if (!(pap > 0.0)) {  // p.Kp <= 0 or NaN: breakdown
-            status = PCG_BREAKDOWN;
-            break;
-        }
+        const bool broke = !(pap > 0.0);  // p.Kp <= 0 or NaN: breakdown
         const double alpha = rz / pap;
         lrr = 0.0;
         lrz = 0.0;
-        if (mine) {
+        if (mine && ok && !broke) {
             r.x -= alpha * q.x;
             r.y -= alpha * q.y;
             const double2 d = ds[t];
@@ -407,7 +433,8 @@ __global__ void __launch_bounds__(T, 1) resident_pcg_kernel(ResidentArgs a) {
             us[t] = u;
         }
         double rz_new;
-        ok = reduce_b(lrr, lrz, unsigned(it) & 1u, rr, rz_new);
+        status = reduce_b(lrr, lrz, ok, broke, unsigned(it) & 1u, rr, rz_new);
+        if (status != PCG_RUNNING) break;
         if (!(rr > surely) && sqrt(rr) / bnorm <= tl) {
             status = PCG_CONVERGED;
         } else if (it >= mi) {
@@ -417,12 +444,12 @@ __global__ void __launch_bounds__(T, 1) resident_pcg_kernel(ResidentArgs a) {
             rz = rz_new;
         }
     }
-    if (!SINGLE && !ok) {
-        // a wait ran out: every CTA of the cluster stops receiving and gets
-        // here, and none leaves while another may still store into it
-        status = RESIDENT_STALLED;
-        cluster_barrier();
-    }
+    // A wait ran out in this CTA.  It has sent nothing since, so the waits of
+    // the others run out in turn, and none leaves while another may still
+    // store into it.  (Others may have ended the solve on the exchange that
+    // came too late here; then the fields are final here too, and they do not
+    // wait for this CTA.)
+    if (!SINGLE && status == RESIDENT_STALLED) cluster_barrier();
     // no CTA's shared memory is written after the last exchange, so the CTAs
     // of a cluster may leave at different times
     if (mine) reinterpret_cast<double2*>(a.u)[N0 + node] = us[t];
@@ -596,12 +623,12 @@ bool resident_shape(const svx_ctx* ctx, int64_t n, int64_t span, bool single,
 void resident_pcg(svx_ctx* ctx, const svx_op* op, const ResidentShape& shape, bool single, cudaStream_t st,
                   int count, const int32_t* order, const int64_t* node_off, const double* tol,
                   const int64_t* max_iter, int64_t* out_it, double* out_res,
-                  int32_t* out_status, double* u) {
+                  int32_t* out_status, double* u, int fault, long long wait_ns) {
     // a single solve takes the registers its thread count leaves free; a
     // batch's CTAs of up to 256 threads share an SM at 128 registers
     const int top = shape.threads <= 256 ? (single ? 256 : MAX_THREADS)
                     : shape.threads <= 384 ? 384 : MAX_THREADS;
-    auto* const kernel =
+    auto* kernel =
         shape.ctas > 1
             ? (top == 256 ? &resident_pcg_kernel<false, 256>
                : top == 384 ? &resident_pcg_kernel<false, 384>
@@ -609,10 +636,6 @@ void resident_pcg(svx_ctx* ctx, const svx_op* op, const ResidentShape& shape, bo
             : (top == 256 ? &resident_pcg_kernel<true, 256>
                : top == 384 ? &resident_pcg_kernel<true, 384>
                             : &resident_pcg_kernel<true, MAX_THREADS>);
-    const void* fn = reinterpret_cast<const void*>(kernel);
-    SVX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  int(RESIDENT_SMEM)));
-    SVX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     ResidentArgs a;
     a.order = order;
     a.node_off = node_off;
@@ -631,6 +654,13 @@ void resident_pcg(svx_ctx* ctx, const svx_op* op, const ResidentShape& shape, bo
     a.out_res = out_res;
     a.out_status = out_status;
     a.window_cap = shape.window;
+    a.wait_ns = fault < 0 ? WAIT_NS : wait_ns;
+    a.fault = fault;
+    if (fault >= 0) kernel = &resident_pcg_kernel<false, MAX_THREADS, true>;
+    const void* fn = reinterpret_cast<const void*>(kernel);
+    SVX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  int(RESIDENT_SMEM)));
+    SVX_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
