@@ -4387,12 +4387,14 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
         stats->fp32_iterations = 0;
         for (int64_t v : f32) stats->fp32_iterations += v;
         stats->ms_solve = ms;
-        // the shape of most members: the resident kernel's, or the autotuned one
-        const bool res = count - n_general > n_small;
-        stats->threads_per_cta = !res ? cfg.bs : op->ndof == 3 ? 256 : ctx->resident_nodes_batch;
-        stats->lanes_per_node = res ? 1 : cfg.g;
-        // the documented classes: 3D >= 4,096 rows, 2D >= 16,384
-        stats->cluster_members = n_large + (op->ndof == 3 ? count - n_general : 0);
+        // the shape of the kernel on the assembled K, whoever runs it
+        stats->threads_per_cta = cfg.bs;
+        stats->lanes_per_node = cfg.g;
+        // members of the documented size (3D >= 4,096 rows, 2D >= 16,384), on
+        // bricks or on K: clusters solve them all
+        stats->cluster_members = 0;
+        for (int k = 0; k < count; ++k)
+            stats->cluster_members += rows_of(k) >= cluster_min_dof(op->ndof);
         stats->member_nnz = std::move(nnz);
     }
 }
