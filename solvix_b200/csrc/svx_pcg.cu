@@ -4307,6 +4307,11 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
                              mixed ? d_fp32.p : nullptr, u_sv, r_sv, p_sv);
         SVX_CUDA(cudaEventRecord(ctx->join_ev, ctx->aux_stream));
     }
+    // the three kinds run side by side: the classes' streams fork before the
+    // one-CTA members are launched, and are joined after
+    const bool classes = n_general < count;
+    if (classes) SVX_CUDA(cudaEventRecord(ctx->fork_ev, pst));
+    if (n_small > 0) launch(choice, d_maxit.p, n_small);
     int n_class = 0;
     for (int k0 = n_general; k0 < count; ++n_class) {
         // the run of members of one shape, its window the largest of them
@@ -4328,7 +4333,6 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
             SVX_CUDA(cudaEventCreateWithFlags(&ce, cudaEventDisableTiming));
             ctx->class_events.push_back(ce);
         }
-        if (n_class == 0) SVX_CUDA(cudaEventRecord(ctx->fork_ev, pst));
         cudaStream_t cs = ctx->class_streams[n_class];
         SVX_CUDA(cudaStreamWaitEvent(cs, ctx->fork_ev, 0));
         if (op->ndof == 3)
@@ -4342,7 +4346,6 @@ void batch_pcg(svx_ctx* ctx, svx_op* op, int count, const std::vector<int64_t>& 
     }
     for (int c = 0; c < n_class; ++c)
         SVX_CUDA(cudaStreamWaitEvent(pst, ctx->class_events[c], 0));
-    if (n_small > 0) launch(choice, d_maxit.p, n_small);
     if (n_large > 0) SVX_CUDA(cudaStreamWaitEvent(pst, ctx->join_ev, 0));
     SVX_CUDA(cudaEventRecord(ctx->ev[1], pst));
     SVX_CUDA(cudaEventRecord(ctx->join_ev, pst));
