@@ -323,9 +323,8 @@ geometry_kernel(BrickView b, int64_t n_elem, const int32_t* __restrict__ conn,
             for (int c = 0; c < 3; ++c) x[a][c] = xyz[3 * nd + c];
         }
         HexModes X(x);
-        const double* m = X.c1;
 #pragma unroll
-        for (int q = 0; q < 21; ++q) geo[q * n_elem + k] = m[q];
+        for (int q = 0; q < 21; ++q) geo[q * n_elem + k] = X.at(q);
 #pragma unroll
         for (int g = 0; g < 8; ++g) {
             double J[3][3];
@@ -476,9 +475,8 @@ __global__ void __launch_bounds__(CH, 1) brick_pcg_kernel(BrickArgs a) {
     auto fetch = [&](int c) {
         const int64_t k = e0 + c * CH + t;
         if (k < e1) {
-            double* m = X.c1;
 #pragma unroll
-            for (int q = 0; q < 21; ++q) m[q] = __ldg(a.geo + q * a.n_elem + k);
+            for (int q = 0; q < 21; ++q) X.at(q) = __ldg(a.geo + q * a.n_elem + k);
 #pragma unroll
             for (int q = 0; q < 10; ++q) late[q] = __ldg(a.geo + (21 + q) * a.n_elem + k);
             lc = __ldg(reinterpret_cast<const uint4*>(b.lconn) + k);
@@ -594,9 +592,8 @@ __global__ void __launch_bounds__(CH, 1) brick_pcg_kernel(BrickArgs a) {
                 const double* g0 = SM ? es + c * CH + t : es + t;
                 if constexpr (SM) {
                     lc = __ldg(reinterpret_cast<const uint4*>(b.lconn) + e0 + c * CH + t);
-                    double* m = X.c1;
 #pragma unroll
-                    for (int q = 0; q < 21; ++q) m[q] = g0[q * held];
+                    for (int q = 0; q < 21; ++q) X.at(q) = g0[q * held];
                     g0 += 21 * held;
                 }
                 double v[8][3];

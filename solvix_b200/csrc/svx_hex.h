@@ -1,13 +1,19 @@
 // svx_hex.h - the C3D8 element operator in registers (device code of
-// svx_hex.cu): trilinear modes, gradients at the Gauss points, forces.
+// svx_hex.cu and svx_brick.cu): trilinear modes, gradients at the Gauss points,
+// forces.  The arithmetic also compiles for the host, where its test runs.
 #ifndef SVX_HEX_H
 #define SVX_HEX_H
 #ifdef __CUDACC__
+#define SVX_HEX_FN __device__ __forceinline__
+#else
+#define SVX_HEX_FN inline
+#endif
 
 namespace svx {
 
 constexpr double HEX_G = 0.57735026918962576450914878050196;  // Gauss abscissa 1 / sqrt(3)
 
+#ifdef __CUDACC__
 __device__ __forceinline__ void load_row(const double* p, double (&v)[3]) {
     [[maybe_unused]] double pad;
     asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
@@ -24,57 +30,60 @@ __device__ __forceinline__ void store_row(double* p, double a, double b, double 
                  "d"(0.0) : "memory");
 }
 
+#endif
+
 // Trilinear modes of eight nodal 3-vectors (corner order element.rs:427-437),
 // eight times the coefficients of xi, eta, zeta, xi eta, eta zeta, xi zeta
 // and xi eta zeta; the products carry their Gauss abscissas (g, g, g, g^2).
 struct HexModes {
-    double c1[3], c2[3], c3[3], c4[3], c5[3], c6[3], c7[3];
+    double c[7][3];  // one array: the bricks store and load all 21 by one index
     HexModes() = default;
-    __device__ __forceinline__ explicit HexModes(const double (&v)[8][3]) {
+    SVX_HEX_FN double& at(int q) { return c[q / 3][q % 3]; }
+    SVX_HEX_FN explicit HexModes(const double (&v)[8][3]) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
+        for (int k = 0; k < 3; ++k) {
             // pairs along xi (0-1, 3-2, 4-5, 7-6), then eta, then zeta
-            const double s0 = v[1][c] + v[0][c], d0 = v[1][c] - v[0][c];
-            const double s1 = v[2][c] + v[3][c], d1 = v[2][c] - v[3][c];
-            const double s2 = v[5][c] + v[4][c], d2 = v[5][c] - v[4][c];
-            const double s3 = v[6][c] + v[7][c], d3 = v[6][c] - v[7][c];
+            const double s0 = v[1][k] + v[0][k], d0 = v[1][k] - v[0][k];
+            const double s1 = v[2][k] + v[3][k], d1 = v[2][k] - v[3][k];
+            const double s2 = v[5][k] + v[4][k], d2 = v[5][k] - v[4][k];
+            const double s3 = v[6][k] + v[7][k], d3 = v[6][k] - v[7][k];
             const double ss0 = s1 + s0, sd0 = s1 - s0, ds0 = d1 + d0, dd0 = d1 - d0;
             const double ss1 = s3 + s2, sd1 = s3 - s2, ds1 = d3 + d2, dd1 = d3 - d2;
-            c1[c] = ds1 + ds0;
-            c2[c] = sd1 + sd0;
-            c3[c] = ss1 - ss0;
-            c4[c] = (dd1 + dd0) * HEX_G;
-            c5[c] = (sd1 - sd0) * HEX_G;
-            c6[c] = (ds1 - ds0) * HEX_G;
-            c7[c] = (dd1 - dd0) * (1.0 / 3.0);
+            c[0][k] = ds1 + ds0;
+            c[1][k] = sd1 + sd0;
+            c[2][k] = ss1 - ss0;
+            c[3][k] = (dd1 + dd0) * HEX_G;
+            c[4][k] = (sd1 - sd0) * HEX_G;
+            c[5][k] = (ds1 - ds0) * HEX_G;
+            c[6][k] = (dd1 - dd0) * (1.0 / 3.0);
         }
     }
-    // G[a][c] = eight times d v_c / d xi_a at Gauss point g (bit 2: xi, 1:
+    // G[a][k] = eight times d v_k / d xi_a at Gauss point g (bit 2: xi, 1:
     // eta, 0: zeta positive)
-    __device__ __forceinline__ void gradient(int g, double (&G)[3][3]) const {
+    SVX_HEX_FN void gradient(int g, double (&G)[3][3]) const {
         const bool x = g & 4, y = g & 2, z = g & 1;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const double a = z ? c1[c] + c6[c] : c1[c] - c6[c];
-            const double b = z ? c4[c] + c7[c] : c4[c] - c7[c];
-            const double d = z ? c2[c] + c5[c] : c2[c] - c5[c];
-            const double e = y ? c3[c] + c5[c] : c3[c] - c5[c];
-            const double f = y ? c6[c] + c7[c] : c6[c] - c7[c];
-            G[0][c] = y ? a + b : a - b;
-            G[1][c] = x ? d + b : d - b;
-            G[2][c] = x ? e + f : e - f;
+        for (int k = 0; k < 3; ++k) {
+            const double a = z ? c[0][k] + c[5][k] : c[0][k] - c[5][k];
+            const double b = z ? c[3][k] + c[6][k] : c[3][k] - c[6][k];
+            const double d = z ? c[1][k] + c[4][k] : c[1][k] - c[4][k];
+            const double e = y ? c[2][k] + c[4][k] : c[2][k] - c[4][k];
+            const double f = y ? c[5][k] + c[6][k] : c[5][k] - c[6][k];
+            G[0][k] = y ? a + b : a - b;
+            G[1][k] = x ? d + b : d - b;
+            G[2][k] = x ? e + f : e - f;
         }
     }
 };
 
-__device__ __forceinline__ double hex_det(const double (&J)[3][3]) {
+SVX_HEX_FN double hex_det(const double (&J)[3][3]) {
     return J[0][0] * (J[1][1] * J[2][2] - J[1][2] * J[2][1]) -
            J[0][1] * (J[1][0] * J[2][2] - J[1][2] * J[2][0]) +
            J[0][2] * (J[1][0] * J[2][1] - J[1][1] * J[2][0]);
 }
 
 // Lame constants over the transforms' powers of two (8^3).
-__device__ __forceinline__ void hex_lame(double E, double nu, double& lam, double& mu) {
+SVX_HEX_FN void hex_lame(double E, double nu, double& lam, double& mu) {
     lam = E * nu / ((1.0 + nu) * (1.0 - 2.0 * nu)) * (1.0 / 512.0);
     mu = E / (2.0 * (1.0 + nu)) * (1.0 / 512.0);
 }
@@ -83,7 +92,7 @@ __device__ __forceinline__ void hex_lame(double E, double nu, double& lam, doubl
 struct HexForces {
     double f1[3], f2[3], f3[3], f4[3], f5[3], f6[3], f7[3];
     // nodal forces from the modes (the transform of HexModes transposed)
-    __device__ __forceinline__ void nodal(double (&f)[8][3]) const {
+    SVX_HEX_FN void nodal(double (&f)[8][3]) const {
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const double m4 = f4[c] * HEX_G, m5 = f5[c] * HEX_G, m6 = f6[c] * HEX_G,
@@ -106,12 +115,12 @@ struct HexForces {
         }
     }
     // u . f over the element (U's products carry g and g^2, the forces not)
-    __device__ __forceinline__ double work(const HexModes& U) const {
+    SVX_HEX_FN double work(const HexModes& U) const {
         double w = 0.0;
 #pragma unroll
         for (int c = 0; c < 3; ++c)
-            w += ((U.c1[c] * f1[c] + U.c2[c] * f2[c]) + (U.c3[c] * f3[c] + U.c4[c] * f4[c])) +
-                 ((U.c5[c] * f5[c] + U.c6[c] * f6[c]) + U.c7[c] * f7[c]);
+            w += ((U.c[0][c] * f1[c] + U.c[1][c] * f2[c]) + (U.c[2][c] * f3[c] + U.c[3][c] * f4[c])) +
+                 ((U.c[4][c] * f5[c] + U.c[5][c] * f6[c]) + U.c[6][c] * f7[c]);
         return w;
     }
 };
@@ -125,7 +134,7 @@ struct HexForces {
 // tenth more operations; it measured 17.0 against 16.4 us an iteration of the
 // whole-device form and 101 against 99 of the graph form).
 template <class R>
-__device__ __forceinline__ void hex_integrate(const HexModes& X, const HexModes& U, double lam,
+SVX_HEX_FN void hex_integrate(const HexModes& X, const HexModes& U, double lam,
                                               double mu, R rdet, HexForces& F) {
 #pragma unroll
     for (int z = 0; z < 2; ++z) {
@@ -213,5 +222,4 @@ __device__ __forceinline__ void hex_integrate(const HexModes& X, const HexModes&
 
 }  // namespace svx
 
-#endif  // __CUDACC__
 #endif  // SVX_HEX_H

@@ -511,7 +511,7 @@ void hex_iteration(const svx_op* op, HexWork& w, cudaStream_t st, const double* 
 
 // Jacobi-PCG of C3D8 models on bricks of elements (svx_brick.cu).
 constexpr int BRICK_LAYERS = 1024;
-constexpr int BRICK_MAX_ELEMS = 2016;        // seven chunks; 16,384 references
+constexpr int BRICK_MAX_ELEMS = 2016;        // eight chunks; 16,128 references
 constexpr size_t BRICK_SMEM = 226 * 1024;    // of 227 KB, less the kernel's static arrays
 struct BrickWork {
     DBuf<double> exchange, part, vec;
