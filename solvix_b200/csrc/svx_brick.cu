@@ -120,11 +120,12 @@ layer_kernel(const int32_t* __restrict__ list, const int64_t* __restrict__ node_
 
 // Elements by layer, in index order within a layer: gridDim.y CTAs a member
 // of the list share its layers (a CTA a layer for a single model; 16 a member
-// of a batch, where most of 1,024 would find an empty layer).
+// of a batch, where most of 1,024 would find an empty layer).  pos, if any,
+// gets each element's place in the order.
 __global__ void __launch_bounds__(256)
 layer_order_kernel(const int32_t* __restrict__ list, const int64_t* __restrict__ elem_off,
                    const uint16_t* __restrict__ layer, const int32_t* __restrict__ hist,
-                   int32_t* __restrict__ order) {
+                   int32_t* __restrict__ order, int32_t* __restrict__ pos) {
     __shared__ int sums[8], base;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int member = list[blockIdx.x];
@@ -145,16 +146,41 @@ layer_order_kernel(const int32_t* __restrict__ list, const int64_t* __restrict__
             const unsigned m = __ballot_sync(0xffffffffu, in);
             if (lane == 0) sums[warp] = __popc(m);
             __syncthreads();
-            int pos = at, all = 0;
+            int rank = at + __popc(m & ((1u << lane) - 1u)), all = 0;
             for (int w = 0; w < 8; ++w) {
-                if (w < warp) pos += sums[w];
+                if (w < warp) rank += sums[w];
                 all += sums[w];
             }
-            if (in) order[e0 + pos + __popc(m & ((1u << lane) - 1u))] = int32_t(e);
+            if (in) {
+                order[e0 + rank] = int32_t(e);
+                if (pos) pos[e] = int32_t(e0 + rank);
+            }
             at += all;
             __syncthreads();
         }
     }
+}
+
+// Nodes of a single model that more than three of its bricks would share
+// (brick k: the elements [n_elem k / bricks, n_elem (k + 1) / bricks) in
+// order), from the pattern's incidence lists.
+__global__ void crowded_kernel(int64_t n_nodes, int64_t n_elem, int64_t bricks,
+                               const int64_t* __restrict__ slot_ptr,
+                               const int32_t* __restrict__ slot_elem,
+                               const int32_t* __restrict__ pos, int* __restrict__ crowded) {
+    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    int n = 0;
+    if (i < n_nodes) {
+        int64_t seen[3] = {-1, -1, -1};
+        for (int64_t s = slot_ptr[i]; s < slot_ptr[i + 1] && n <= 3; ++s) {
+            const int64_t k = ((int64_t(pos[slot_elem[s]]) + 1) * bricks - 1) / n_elem;
+            if (k == seen[0] || k == seen[1] || k == seen[2]) continue;
+            if (n < 3) seen[n] = k;
+            ++n;
+        }
+    }
+    const int many = __syncthreads_count(n > 3);
+    if (threadIdx.x == 0 && many) atomicAdd(crowded, many);
 }
 
 __device__ void bitonic(uint32_t* key, int m) {
@@ -282,20 +308,18 @@ brick_build_kernel(BrickView b, const int32_t* __restrict__ conn, int32_t* ent_n
     }
 }
 
-// Every node's entries in ascending brick order, and how many nodes more than
-// three bricks share; gridDim.y CTAs a member of the list.
+// Every node's entries in ascending brick order; gridDim.y CTAs a member of
+// the list.
 __global__ void entry_sort_kernel(const int32_t* __restrict__ list,
                                   const int64_t* __restrict__ node_off,
                                   uint32_t* __restrict__ entry,
-                                  const int32_t* __restrict__ ent_n, int* __restrict__ fail,
-                                  int* __restrict__ crowded) {
+                                  const int32_t* __restrict__ ent_n, int* __restrict__ fail) {
     const int member = list[blockIdx.x];
     const int64_t n1 = node_off[member + 1];
     for (int64_t i = node_off[member] + int64_t(blockIdx.y) * blockDim.x + threadIdx.x;
          i < n1; i += int64_t(gridDim.y) * blockDim.x) {
         const int n = min(ent_n[i], SHARE);
         if (n == 0) fail[member] = 1;
-        if (n > 3) atomicAdd(&crowded[member], 1);
         uint32_t* e = entry + i * SHARE;
         for (int a = 1; a < n; ++a) {
             const uint32_t v = e[a];
@@ -865,7 +889,7 @@ void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_
     B.bricks = bricks;
     DBuf<int64_t> d_noff, d_eoff;
     DBuf<uint16_t> layer;
-    DBuf<int32_t> hist, ent_n, d_list;
+    DBuf<int32_t> hist, ent_n, d_list, pos;
     DBuf<int> fail;
     const unsigned listed = unsigned(list.size());
     d_noff.alloc(ctx->pool, members + 1);
@@ -873,9 +897,46 @@ void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_
     layer.alloc(ctx->pool, size_t(op->n_elem));
     d_list.alloc(ctx->pool, listed);
     hist.alloc(ctx->pool, size_t(listed) * BRICK_LAYERS);
-    ent_n.alloc(ctx->pool, size_t(op->n_nodes));
-    fail.alloc(ctx->pool, 2 * size_t(members));  // and the nodes many bricks share
+    if (single) pos.alloc(ctx->pool, size_t(op->n_elem));
+    fail.alloc(ctx->pool, size_t(members) + 1);  // and the nodes many bricks share
     B.order.alloc(ctx->pool, size_t(op->n_elem));
+    auto up = [&](auto& dst, const auto& src) {
+        SVX_CUDA(cudaMemcpyAsync(dst.p, src.data(), src.size() * sizeof(src[0]),
+                                 cudaMemcpyHostToDevice, st));
+    };
+    std::vector<int> bad(size_t(members) + 1);
+    auto read_back = [&]() {
+        SVX_CUDA(cudaMemcpyAsync(bad.data(), fail.p, sizeof(int) * bad.size(),
+                                 cudaMemcpyDeviceToHost, st));
+        SVX_CUDA(cudaStreamSynchronize(st));
+    };
+    up(d_noff, node_off);
+    up(d_eoff, elem_off);
+    up(d_list, list);
+    SVX_CUDA(cudaMemsetAsync(hist.p, 0, sizeof(int32_t) * size_t(listed) * BRICK_LAYERS, st));
+    SVX_CUDA(cudaMemsetAsync(fail.p, 0, sizeof(int) * bad.size(), st));
+    layer_kernel<<<listed, 1024, 0, st>>>(d_list.p, d_noff.p, d_eoff.p, op->conn.p, op->xyz.p,
+                                          layer.p, hist.p);
+    SVX_LAUNCH_CHECK();
+    layer_order_kernel<<<dim3(listed, single ? BRICK_LAYERS : 16), 256, 0, st>>>(
+        d_list.p, d_eoff.p, layer.p, hist.p, B.order.p, pos.p);
+    SVX_LAUNCH_CHECK();
+    // A model whose layers take several bricks has nodes that four and more
+    // bricks share; their sums go through the lists in global memory.  A 35^3
+    // cube runs 27.0 us an iteration that way and 19.7 on its assembled K.  The
+    // element order alone tells, so such a model is left before anything is built.
+    if (single) {
+        crowded_kernel<<<unsigned((op->n_nodes + 255) / 256), 256, 0, st>>>(
+            op->n_nodes, op->n_elem, bricks, op->pat.slot_ptr.p, op->pat.slot_elem.p, pos.p,
+            fail.p + members);
+        SVX_LAUNCH_CHECK();
+        read_back();
+        if (bad[members] > op->n_nodes / 50) {
+            nbricks[0] = 0;
+            return;
+        }
+    }
+    ent_n.alloc(ctx->pool, size_t(op->n_nodes));
     B.elem0.alloc(ctx->pool, bricks);
     B.elem1.alloc(ctx->pool, bricks);
     B.member.alloc(ctx->pool, bricks);
@@ -889,27 +950,12 @@ void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_
     B.ccount.alloc(ctx->pool, chunks);
     B.entry.alloc(ctx->pool, size_t(op->n_nodes) * SHARE);
     B.geo.alloc(ctx->pool, size_t(op->n_elem) * GEO);
-    auto up = [&](auto& dst, const auto& src) {
-        SVX_CUDA(cudaMemcpyAsync(dst.p, src.data(), src.size() * sizeof(src[0]),
-                                 cudaMemcpyHostToDevice, st));
-    };
-    up(d_noff, node_off);
-    up(d_eoff, elem_off);
-    up(d_list, list);
     up(B.elem0, e0);
     up(B.elem1, e1);
     up(B.member, bm);
     up(B.chunk0, c0);
     up(B.member_brick, mb);
-    SVX_CUDA(cudaMemsetAsync(hist.p, 0, sizeof(int32_t) * size_t(listed) * BRICK_LAYERS, st));
     SVX_CUDA(cudaMemsetAsync(ent_n.p, 0, sizeof(int32_t) * size_t(op->n_nodes), st));
-    SVX_CUDA(cudaMemsetAsync(fail.p, 0, sizeof(int) * 2 * size_t(members), st));
-    layer_kernel<<<listed, 1024, 0, st>>>(d_list.p, d_noff.p, d_eoff.p, op->conn.p, op->xyz.p,
-                                          layer.p, hist.p);
-    SVX_LAUNCH_CHECK();
-    layer_order_kernel<<<dim3(listed, single ? BRICK_LAYERS : 16), 256, 0, st>>>(
-        d_list.p, d_eoff.p, layer.p, hist.p, B.order.p);
-    SVX_LAUNCH_CHECK();
     const size_t bsm = size_t(SORT_BRICK + ncap) * 4;
     SVX_CUDA(cudaFuncSetAttribute(reinterpret_cast<const void*>(&brick_build_kernel),
                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -917,18 +963,12 @@ void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_
     brick_build_kernel<<<bricks, BT, bsm, st>>>(B.view(), op->conn.p, ent_n.p, fail.p);
     SVX_LAUNCH_CHECK();
     entry_sort_kernel<<<dim3(listed, single ? 256 : 16), 256, 0, st>>>(
-        d_list.p, d_noff.p, B.entry.p, ent_n.p, fail.p, fail.p + members);
+        d_list.p, d_noff.p, B.entry.p, ent_n.p, fail.p);
     SVX_LAUNCH_CHECK();
     brick_constants(ctx, op);
-    std::vector<int> bad(2 * size_t(members));
-    SVX_CUDA(cudaMemcpyAsync(bad.data(), fail.p, sizeof(int) * bad.size(),
-                             cudaMemcpyDeviceToHost, st));
-    SVX_CUDA(cudaStreamSynchronize(st));
-    // A model whose layers take several bricks has nodes that four and more
-    // bricks share; their sums go through the lists in global memory.  A 35^3
-    // cube runs 27.0 us an iteration that way and 19.7 on its assembled K.
+    read_back();
     for (int m = 0; m < members; ++m)
-        if (bad[m] || (single && bad[members + m] > op->n_nodes / 50)) nbricks[m] = 0;
+        if (bad[m]) nbricks[m] = 0;
 }
 
 namespace {

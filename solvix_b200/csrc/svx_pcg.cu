@@ -3225,6 +3225,7 @@ static void wire_hex_form(svx_ctx* ctx, svx_op* op, PcgRun<double, double, doubl
         std::vector<int> nbricks{coop && per <= ctx->brick_max_elems
                                      ? int((op->n_elem + per - 1) / per) : 0};
         if (nbricks[0] > 0) brick_build(ctx, op, true, {0, op->n_nodes}, {0, op->n_elem}, nbricks);
+        if (nbricks[0] == 0) op->brick = BrickOperator{};  // what was built goes back
         op->brick.state = nbricks[0] > 0 ? 1 : -1;
     }
     if (op->brick.state > 0) {
