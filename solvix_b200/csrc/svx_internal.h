@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "solvix_gpu.h"
+#include "svx_pinned.h"
 
 namespace svx {
 
@@ -122,38 +123,24 @@ struct DBuf {
     size_t bytes() const { return n * sizeof(T); }
 };
 
-// Growable page-locked host buffer (one per context) that stages batched
-// uploads and downloads, so they run as single DMA copies.  Contents are
-// valid until the next get(); callers synchronise their stream first.
-class PinnedBuffer {
+// The page-locked buffer (one per context) that stages uploads and downloads,
+// so they run as single DMA copies.
+struct CudaHost {
+    static void* alloc(size_t bytes) {
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, bytes, cudaHostAllocDefault) == cudaSuccess) return p;
+        cudaGetLastError();
+        return nullptr;
+    }
+    static void free(void* p) { cudaFreeHost(p); }
+};
+class PinnedBuffer : public PinnedBufferT<CudaHost> {
 public:
-    PinnedBuffer() = default;
-    PinnedBuffer(const PinnedBuffer&) = delete;
-    PinnedBuffer& operator=(const PinnedBuffer&) = delete;
-    ~PinnedBuffer() {
-        if (p_) cudaFreeHost(p_);
-    }
     void* get(size_t bytes) {
-        if (bytes > cap_) {
-            if (p_) cudaFreeHost(p_);
-            p_ = nullptr;
-            cap_ = 0;
-            size_t want = size_t(1) << 20;  // sizes double, so a growing series allocates rarely
-            while (want < bytes) want *= 2;
-            cudaError_t e = cudaHostAlloc(&p_, want, cudaHostAllocDefault);
-            if (e != cudaSuccess) {
-                cudaGetLastError();
-                p_ = nullptr;
-                throw ModelFail{SVX_OOM, 0, -1, "page-locked host allocation failed"};
-            }
-            cap_ = want;
-        }
-        return p_;
+        void* p = try_get(bytes);
+        if (!p) throw ModelFail{SVX_OOM, 0, -1, "page-locked host allocation failed"};
+        return p;
     }
-
-private:
-    void* p_ = nullptr;
-    size_t cap_ = 0;
 };
 
 }  // namespace svx
