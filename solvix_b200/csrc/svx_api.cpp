@@ -361,11 +361,12 @@ constexpr size_t STAGE_MAX = size_t(256) << 20;
 
 // Uploads through the context's staging buffer, which must be idle (every call
 // that used it has waited for its stream) and holds them until the next wait;
-// without room (bytes = 0) the copies run from the caller's memory.
+// without one (bytes = 0, or the host refuses it) the copies run from the
+// caller's memory.
 class Stager {
 public:
     Stager(svx_ctx* ctx, size_t bytes)
-        : ctx_(ctx), at_(bytes ? static_cast<char*>(ctx->staging.get(bytes)) : nullptr) {}
+        : ctx_(ctx), at_(bytes ? static_cast<char*>(ctx->staging.try_get(bytes)) : nullptr) {}
     template <class T>
     void upload(DBuf<T>& dst, const T* src, size_t count) {
         if (at_ && count) {
@@ -651,12 +652,13 @@ void stress_to_device(svx_op* op) {
 
 // Results to the caller's arrays: through the idle staging buffer, so that the
 // copies run as DMA behind one another, and from there after the wait
-// (finish()); sets too large for it are copied as they lie.
+// (finish()); sets too large for it, or for the host, are copied as they lie.
 class Fetcher {
 public:
     Fetcher(svx_ctx* ctx, size_t bytes)
         : ctx_(ctx),
-          at_(bytes <= STAGE_MAX ? static_cast<char*>(ctx->staging.get(bytes + 1024)) : nullptr) {}
+          at_(bytes <= STAGE_MAX ? static_cast<char*>(ctx->staging.try_get(bytes + 1024))
+                                 : nullptr) {}
     void add(double* to, const double* from, int64_t count) {
         if (!to || count <= 0) return;
         const size_t bytes = size_t(count) * sizeof(double);
@@ -1064,6 +1066,11 @@ int svx_ctx_create(int device, svx_ctx_t** out) {
             char* end = nullptr;
             const long long v = std::strtoll(e, &end, 10);
             if (end != e && v >= 0) ctx->graph_min_nnz = v;
+        }
+        if (const char* e = std::getenv("SVX_STAGING_MAX")) {
+            char* end = nullptr;
+            const long long v = std::strtoll(e, &end, 10);
+            if (end != e && v >= 0) ctx->staging.limit = size_t(v);
         }
         if (const char* e = std::getenv("SVX_PCG_SMEM")) ctx->pcg_smem = (e[0] != '0');
         if (const char* e = std::getenv("SVX_PCG_ALG")) ctx->pcg_alg = (e[0] == '0') ? 0 : 1;
