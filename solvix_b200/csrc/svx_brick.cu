@@ -242,7 +242,8 @@ brick_build_kernel(BrickView b, const int32_t* __restrict__ conn, int32_t* ent_n
     for (int q = q0; q < q1; ++q) count += q == 0 || key[q] != key[q - 1];
     int nn;
     int at = block_scan(count, sh, nn);
-    if (nn > b.ncap) {
+    const uint32_t base = b.node0[brick];
+    if (nn > int(b.node0[brick + 1] - base)) {
         if (threadIdx.x == 0) fail[b.member[brick]] = 1;
         return;
     }
@@ -252,9 +253,9 @@ brick_build_kernel(BrickView b, const int32_t* __restrict__ conn, int32_t* ent_n
     if (threadIdx.x == 0) b.count[brick] = nn;
     for (int l = threadIdx.x; l < nn; l += BT) {
         const uint32_t nd = node[l];
-        b.node[int64_t(brick) * b.ncap + l] = int32_t(nd);
+        b.node[base + l] = int32_t(nd);
         const int k = atomicAdd(&ent_n[nd], 1);
-        if (k < SHARE) b.entry[int64_t(nd) * SHARE + k] = uint32_t(brick) * uint32_t(b.ncap) + l;
+        if (k < SHARE) b.entry[int64_t(nd) * SHARE + k] = base + uint32_t(l);
         else fail[b.member[brick]] = 1;
     }
     for (int q = threadIdx.x; q < refs; q += BT) {
@@ -388,7 +389,7 @@ struct BrickArgs {
     const double* f;          // batch: right-hand side
     double *u, *r, *p;        // node vectors (grid: state between launches)
     double *rb, *ub, *db;     // bricks' copies of r, u, 1 / K_ii (vectors not in shared memory)
-    double* rows;             // [2][bricks * ncap][4] partial forces, in turn
+    double* rows;             // [2][slots][4] partial forces, in turn
     double* part;             // [3][bricks] sums of each brick: p.Kp, then r.r and r.z
     // grid
     PcgScalars* s;
@@ -431,7 +432,9 @@ __global__ void __launch_bounds__(CH, 1) brick_pcg_kernel(BrickArgs a) {
     }
     const int e0 = b.elem0[brick], e1 = b.elem1[brick];
     const int nn = b.count[brick];
-    const int64_t base = int64_t(brick) * b.ncap;
+    // (read from memory, a single model's would cost this kernel 130 bytes of
+    // spills and a tenth of its time)
+    const int64_t base = GRID ? int64_t(brick) * b.ncap : int64_t(b.node0[brick]);
     const int chunks = (e1 - e0 + CH - 1) / CH;
     // shared memory: staged forces, element constants, force sums (of all
     // chunks in SM, of one otherwise), p, q (and r, u, 1 / K_ii),
@@ -601,7 +604,7 @@ __global__ void __launch_bounds__(CH, 1) brick_pcg_kernel(BrickArgs a) {
     if (surely < 1e-280) surely = INFINITY;  // the square left the normal range
     __syncthreads();
     for (int step = 0; status == PCG_RUNNING && (!GRID || step < a.chunk); ++step) {
-        const int64_t turn_at = (step & 1) * int64_t(b.bricks) * b.ncap;
+        const int64_t turn_at = (step & 1) * (GRID ? int64_t(b.bricks) * b.ncap : b.slots);
         double* rows = a.rows + 4 * turn_at;
         auto share = [&](int l, const double (&q)[3]) {
             store_row(rows + 4 * (base + l), q[0], q[1], q[2]);
@@ -887,6 +890,12 @@ void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_
     B.lists = single ? lists_of(ncap) : 1 << 30;
     B.ncap = ncap;
     B.bricks = bricks;
+    // slots of the bricks' nodes: in a batch, a brick of few elements takes
+    // few, whatever the largest takes; a single model's bricks are alike
+    std::vector<uint32_t> n0(1, 0);
+    for (int k = 0; k < bricks; ++k)
+        n0.push_back(n0.back() + uint32_t(single ? ncap : std::min(ncap, 8 * (e1[k] - e0[k]))));
+    B.slots = n0.back();
     DBuf<int64_t> d_noff, d_eoff;
     DBuf<uint16_t> layer;
     DBuf<int32_t> hist, ent_n, d_list, pos;
@@ -943,7 +952,8 @@ void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_
     B.chunk0.alloc(ctx->pool, bricks);
     B.member_brick.alloc(ctx->pool, members + 1);
     B.lconn.alloc(ctx->pool, size_t(op->n_elem) * 8);
-    B.node.alloc(ctx->pool, size_t(bricks) * ncap);
+    B.node0.alloc(ctx->pool, bricks + 1);
+    B.node.alloc(ctx->pool, size_t(B.slots));
     B.count.alloc(ctx->pool, bricks);
     B.ref.alloc(ctx->pool, size_t(chunks) * CN * 8);
     B.cnode.alloc(ctx->pool, size_t(chunks) * CN);
@@ -954,6 +964,7 @@ void brick_build(svx_ctx* ctx, svx_op* op, bool single, const std::vector<int64_
     up(B.elem1, e1);
     up(B.member, bm);
     up(B.chunk0, c0);
+    up(B.node0, n0);
     up(B.member_brick, mb);
     SVX_CUDA(cudaMemsetAsync(ent_n.p, 0, sizeof(int32_t) * size_t(op->n_nodes), st));
     const size_t bsm = size_t(SORT_BRICK + ncap) * 4;
@@ -983,7 +994,7 @@ BrickArgs brick_args(const svx_op* op, BrickWork& w) {
     a.part = w.part.p;
     a.rb = w.vec.p;
     if (w.vec.p) {
-        const size_t n = size_t(op->brick.bricks) * op->brick.ncap * 3;
+        const size_t n = size_t(op->brick.slots) * 3;
         a.ub = w.vec.p + n;
         a.db = w.vec.p + 2 * n;
     }
@@ -993,9 +1004,9 @@ BrickArgs brick_args(const svx_op* op, BrickWork& w) {
 
 void BrickWork::alloc(svx_ctx* ctx, const svx_op* op, bool single) {
     const BrickOperator& B = op->brick;
-    exchange.alloc(ctx->pool, size_t(B.bricks) * B.ncap * 8);
+    exchange.alloc(ctx->pool, size_t(B.slots) * 8);
     part.alloc(ctx->pool, size_t(B.bricks) * 3 + 4);
-    if (!single) vec.alloc(ctx->pool, size_t(B.bricks) * B.ncap * 9);
+    if (!single) vec.alloc(ctx->pool, size_t(B.slots) * 9);
     gb.alloc(ctx->pool, 1);
 }
 

@@ -292,16 +292,18 @@ struct HexOperator {
 
 // The bricks of C3D8 models (svx_brick.cu).
 struct BrickView {
-    int bricks, ncap;              // ncap: nodes a brick may have
+    int bricks, ncap;              // ncap: nodes a brick may have in shared memory
     int held, lists;               // elements and chunk nodes held in shared memory
+    int64_t slots;                 // node0[bricks]
+    const uint32_t* node0;         // [bricks + 1] its node slots (room by its elements)
     const int32_t *elem0, *elem1;  // [bricks] its elements, positions in `order`
     const int32_t* member;         // [bricks]
     const int32_t* chunk0;         // [bricks] its first chunk
     const int32_t* order;          // [n_elem] elements by layer
     int32_t* count;                // [bricks] nodes
-    int32_t* node;                 // [bricks][ncap]
+    int32_t* node;                 // [slots]
     uint16_t* lconn;               // [n_elem][8] nodes of the brick, in `order`
-    uint32_t* entry;               // [n_nodes][8] brick * ncap + place, ascending (~0: none)
+    uint32_t* entry;               // [n_nodes][8] node slots, ascending (~0: none)
     // per chunk: its nodes (places in the brick), and eight offsets of staged
     // forces for each, in ascending element order
     uint16_t *cnode, *ref;
@@ -311,13 +313,16 @@ struct BrickOperator {
     int bricks = 0, ncap = 0, held = 0, lists = 0;
     int state = 0;     // single models: 0 not built, 1 built, -1 does not fit
     bool stale = false;  // geo is older than the last assembly (the lists are not)
+    int64_t slots = 0;
+    DBuf<uint32_t> node0;
     DBuf<int32_t> elem0, elem1, member, chunk0, order, count, node, ccount, member_brick;
     DBuf<uint16_t> lconn, cnode, ref;
     DBuf<uint32_t> entry;
     DBuf<double> geo;
     BrickView view() const {
-        return BrickView{bricks,  ncap,   held,    lists,   elem0.p, elem1.p, member.p, chunk0.p,
-                         order.p, count.p, node.p, lconn.p, entry.p, cnode.p, ref.p,    ccount.p};
+        return BrickView{bricks,   ncap,    held,    lists,  slots,   node0.p,
+                         elem0.p,  elem1.p, member.p, chunk0.p, order.p, count.p,
+                         node.p,   lconn.p, entry.p, cnode.p, ref.p,   ccount.p};
     }
 };
 
