@@ -288,10 +288,10 @@ void apply_dirichlet(svx_ctx* ctx, svx_op* op) {
         op->kc_ptr.alloc(ctx->pool, m + 1);
         fixed_ptr_kernel<<<1, 1024, 0, st>>>(m, op->fixed_uniq.p, P.row_ptr.p, op->kc_ptr.p);
         SVX_LAUNCH_CHECK();
-        // room for every row at the largest degree, where that is small, saves
-        // the wait for the rows' own total
+        // room for every row at the largest degree, where that is small (12 MB),
+        // saves the wait for the rows' own total
         int64_t room = m * int64_t(op->ndof) * std::max(1, P.max_deg);
-        if (room > (int64_t(1) << 26)) {
+        if (room > (int64_t(1) << 20)) {
             int32_t total = 0;
             SVX_CUDA(cudaMemcpyAsync(&total, op->kc_ptr.p + m, sizeof(total),
                                      cudaMemcpyDeviceToHost, st));
