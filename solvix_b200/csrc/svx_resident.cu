@@ -41,6 +41,7 @@
 // largest members ran alone at the end).
 
 #include "svx_internal.h"
+#include "svx_quotient.h"
 #include "svx_warp.h"
 
 #include <cmath>
@@ -141,16 +142,6 @@ __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity,
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-}
-
-// x / y from y's reciprocal: one residual correction brings the product to
-// within an ulp of the quotient (Markstein 1990); operands outside the range
-// where the residual is exact take the division.
-__device__ __forceinline__ double quotient(double x, double y, double y_inv) {
-    const double ay = fabs(y), ax = fabs(x);
-    if (!(ay > 1e-140 && ay < 1e140 && ax > 1e-140 && ax < 1e140)) return x / y;
-    const double q = x * y_inv;
-    return __fma_rn(__fma_rn(-y, q, x), y_inv, q);
 }
 
 // What the CTAs of a cluster write into each other.
