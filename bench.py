@@ -13,9 +13,9 @@ of 1e-10 and von Mises / reaction recovery.
   (svx_solve_flat) from pinned host buffers: the model's H2D copy and the
   D2H read of u, displacements, von Mises and reactions are inside the
   timed region.
-* ``roofline`` - the dominant kernel (the persistent PCG kernel) against
-  the measured HBM copy peak, from its algorithmic bytes and its live
-  CUDA-event duration.
+* ``roofline`` - the dominant kernel (the persistent element-by-element PCG
+  kernel) against the FP64 rate, from its operations and its live CUDA-event
+  duration, and the standalone SpMV against the measured HBM copy peak.
 * ``cpu_baseline`` - the oracle (the C++ restatement of the reference's
   Rust path) solving the same model on the host cores.
 * ``precision_c3``, ``batched_c4``, ``served_c5`` - the metric's own
@@ -314,19 +314,21 @@ def run_ours(args, rank, world, local_rank):
     dof_iters = float(np.sum(iters)) * n
     value = world * dof_iters / (ms_max / 1000.0)
 
-    # roofline of the dominant kernel, the persistent PCG kernel: the
-    # algorithmic bytes of PCG on the assembled K per launch (CHUNK iterations) over its average
-    # launch duration, from the PCG device time of the timed steps
-    from solvix_b200.roofline import pcg_iteration_bytes, spmv_node_bytes
+    # roofline of the dominant kernel, the persistent PCG kernel, per launch
+    # (CHUNK iterations) over its average duration, from the PCG device time of
+    # the timed steps: the FP64 operations of its elements
+    from solvix_b200.roofline import hex_iteration_flops, spmv_node_bytes
     # iterations per persistent launch (persistent_chunk in svx_pcg.cu)
     chunk = 64 if nnz > 100_000_000 else (256 if nnz > 10_000_000 else 1024)
     it_total = float(np.sum(iters))
     launches_pcg = float(sum(-(-i // chunk) for i in iters))
-    iter_bytes = pcg_iteration_bytes(n, nnz, flat.ndof, flat.n_nodes)
+    iter_flops = hex_iteration_flops(flat.n_elem, flat.n_nodes)
     launch_ms = ms_parts[1] / launches_pcg
-    launch_bytes = iter_bytes * it_total / launches_pcg
-    achieved = launch_bytes / (launch_ms / 1000.0) / 1e9
-    peak, peak_kind = measured_peaks()
+    launch_flops = iter_flops * it_total / launches_pcg
+    achieved = launch_flops / (launch_ms / 1000.0) / 1e12
+    peak, _ = measured_peaks()
+    sms = torch.cuda.get_device_properties(local_rank).multi_processor_count
+    fp64_peak = sms * 64 * 2 * 1.965e9 / 1e12
     traffic_it = ncu_traffic()
     traffic = traffic_it * it_total / launches_pcg if traffic_it else None
     # the node-block SpMV alone (spmv_node_dot), back-to-back launches
@@ -406,18 +408,19 @@ def run_ours(args, rank, world, local_rank):
                 "d2h_bytes_per_step": int(d2h), "steps": e2e_steps,
                 "solves_per_s": world * e2e_steps / (float(e_ms.item()) / 1000.0)},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": "brick_pcg_kernel (FP64, element by element, "
-                                                 f"{chunk} PCG iterations a launch)",
-                     "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak, "peak_source": peak_kind,
-                     "algorithmic_bytes_per_launch": int(launch_bytes),
-                     "algorithmic_bytes_per_iteration": int(iter_bytes),
+        "roofline": {"bound": "fp64", "kernel": "brick_pcg_kernel (FP64, element by element, "
+                                                  f"{chunk} PCG iterations a launch)",
+                     "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s",
+                     "frac": achieved / fp64_peak,
+                     "peak_source": "nominal (64 FP64 FMA a clock and SM at 1,965 MHz; no "
+                                    "measured FP64 peak exists)",
+                     "flops_per_launch": int(launch_flops),
+                     "flops_per_iteration": int(iter_flops),
                      "launch_ms": float(launch_ms),
                      "traffic": traffic,
-                     "note": "the algorithmic bytes are an iteration's on the assembled K (87.7 "
-                             "MB), which this kernel does not read: it forms K p from the "
-                             "elements, with its constants and vectors on the chip, so the "
-                             "rate can exceed the copy peak",
+                     "note": "K p is formed from the elements, whose constants and vectors stay "
+                             "on the chip; the rest of an iteration is two sums over the grid "
+                             "and the latency of an element's chain at 8 warps an SM",
                      "spmv_node_dot_alone": {
                          "launch_ms": float(kms[0]), "bytes": int(spmv_bytes),
                          "gbs": spmv_bytes / (kms[0] / 1000.0) / 1e9,
