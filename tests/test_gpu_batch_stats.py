@@ -10,6 +10,14 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.fixture(scope="module")
+def fresh():
+    """A context of its own: the session's may have its CTA shape autotuned."""
+    c = Context(0)
+    yield c
+    c.close()
+
+
+@pytest.fixture(scope="module")
 def on_k():
     old = {k: os.environ.get(k) for k in ("SVX_HEX", "SVX_RESIDENT")}
     os.environ.update({k: "0" for k in old})
@@ -33,10 +41,10 @@ def plates():
 
 
 @pytest.mark.parametrize("flats,clusters", [(hexes, 1), (plates, 0)])
-def test_statistics_are_those_of_the_assembled_form(ctx, on_k, flats, clusters):
+def test_statistics_are_those_of_the_assembled_form(fresh, on_k, flats, clusters):
     flats = flats()
     assert sum(f.n_dof >= (4096 if f.ndof == 3 else 16384) for f in flats) == clusters
-    _, new = ctx.solve_batch(flats)
+    _, new = fresh.solve_batch(flats)
     _, old = on_k.solve_batch(flats)
     for name in ("cluster_members", "threads_per_cta", "lanes_per_node", "total_dof"):
         assert new[name] == old[name], name
