@@ -566,6 +566,8 @@ def run_batched(args, rank, world, local_rank):
         "roofline": {"bound": "hbm", "kernel": "FP64: resident_pcg_kernel (one cluster per plate, K "
                                                  "in registers), one launch a size class; mixed: "
                                                  "batch_pcg_mixed_kernel",
+                     "note": "bytes of PCG on the assembled K, which only the mixed form streams: "
+                             "in FP64 the rate compares with it and is no share of the peak",
                      "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": peak_kind,
                      "algorithmic_bytes_per_launch": int(bytes_alg),
@@ -835,14 +837,16 @@ def run_served(args, rank, world, local_rank):
                 "h2d_bytes_per_step": int(sum(f.nbytes() for f in reqs)),
                 "d2h_bytes_per_step": int(sum(8 * (f.n_dof + f.n_elem) for f in reqs))},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": "batch_pcg_kernel / batch_pcg_cluster_kernel "
-                     "of every lane's batches",
+        "roofline": {"bound": "hbm", "kernel": "every lane's batches; FP64: resident_pcg_kernel and "
+                     "brick_pcg_kernel, mixed: batch_pcg_mixed_kernel and "
+                     "batch_pcg_cluster_kernel",
                      "achieved": sat["algorithmic_bytes"] / sat["wall_s"] / 1e9,
                      "peak": peak, "unit": "GB/s",
                      "frac": sat["algorithmic_bytes"] / sat["wall_s"] / 1e9 / peak,
                      "peak_source": peak_kind,
                      "algorithmic_bytes": sat["algorithmic_bytes"],
-                     "note": "over the saturation run's wall clock, host phases included",
+                     "note": "over the saturation run's wall clock, host phases included; bytes "
+                             "of PCG on the assembled K, which only the mixed form streams",
                      "traffic": None},
         "clocks": clk,
     }
